@@ -133,6 +133,8 @@ wt::StepArgs<S> make_args(wt_lattice* h) {
   a.n = h->n;
   a.nxy = (long long)h->nx * h->ny;
   const bool narrow = 19 * h->n * (long long)sizeof(S) < (1LL << 31);
+  a.row = wt::fast_div((unsigned)wt::row_cells(h->nx));
+  a.zfast = h->stats.ground && (double)h->n * 19 * sizeof(S) <= (double)h->l2 ? 1 : 0;
   for (int q = 0; q < 19; q++) {
     const long long off = wt::ex(q) + (long long)h->nx * wt::ey(q) + a.nxy * wt::ez(q);
     a.src[q] = q * h->n - off;
@@ -185,7 +187,7 @@ void run_steps(wt_lattice* h, int nsteps, StepLaunch<S> launch, double* part, do
                unsigned* err, int chunk_max) {
   wt::StepArgs<S> a = make_args<S>(h);
   a.err = err;
-  const dim3 grid = wt::step_grid(h->nx, h->ny, h->nz);
+  const dim3 grid = wt::step_grid(a);
   const bool wide = 19 * h->n >= (1LL << 31);
   const size_t stride = 3 * (size_t)h->nslots;
   for (int done = 0; done < nsteps;) {
@@ -209,15 +211,17 @@ void run_steps(wt_lattice* h, int nsteps, StepLaunch<S> launch, double* part, do
 
 bool lean_ok(const wt_lattice* h);
 bool pair_ok(const wt_lattice* h);
+bool pair_auto(const wt_lattice* h);
 
 // The kernel WT_KERNEL_AUTO runs, the fastest measured on B200 for the form
 // (256x128x128 channel, 1000-step calls): the pair kernel where it can run
 // (float32 storage 40.3k MLUPS against 37.9k for the lean kernel; half
-// storage 55.2k against 44.4k), the lean kernel for an odd nx, the direct
-// kernel otherwise (exact collision, float64, moving walls, buffers of 2^31
+// storage 55.2k against 44.4k; odd nx and moving walls: PAIR_ODD, PAIR_MOV),
+// the lean kernel for half storage with an odd nx, the direct kernel otherwise
+// (exact collision, float64, half storage with moving walls, buffers of 2^31
 // bytes or more).
 Path auto_path(const wt_lattice* h) {
-  if (pair_ok(h)) return Path::Pair;
+  if (pair_auto(h)) return Path::Pair;
   if (lean_ok(h)) return Path::Lean;
   return Path::Direct;
 }
@@ -235,6 +239,14 @@ bool lean_ok(const wt_lattice* h) {
 // collision, so half or float32 storage) and an even nx (aligned pairs of
 // cells).
 bool pair_ok(const wt_lattice* h) { return lean_ok(h) && h->nx % 2 == 0; }
+
+// True when AUTO takes the pair kernel: besides the lattices that may ask for
+// it, float32 storage with an odd nx or moving walls (PAIR_ODD, PAIR_MOV).
+bool pair_auto(const wt_lattice* h) {
+  if (pair_ok(h)) return true;
+  return h->storage == WT_STORE_F32 && h->p.math != WT_MATH_EXACT &&
+         19 * h->n * (long long)h->elem < (1LL << 31);
+}
 
 int select_path(wt_lattice* h, Path* out);
 void dispatch_steps(wt_lattice* h, int nsteps, Path path, double* part, double* forces_dev,
@@ -261,11 +273,11 @@ int rebuild_slots(wt_lattice* h) {
   if (h->sfrac) {
     // every segment that touches the partial bounce-back box carries a force partial
     const int* b = h->sbox;
-    const int nseg = (h->nx + 31) / 32;
     for (int z = b[2]; z < b[5]; z++)
-      for (int y = b[1]; y < b[4]; y++)
-        for (int sx = b[0] / 32; sx <= (b[3] - 1) / 32; sx++)
-          hm[((size_t)z * h->ny + y) * nseg + sx] = 1;
+      for (int y = b[1]; y < b[4]; y++) {
+        const long long s1 = wt::seg_of(b[3] - 1, y, z, h->nx, h->ny);
+        for (long long s = wt::seg_of(b[0], y, z, h->nx, h->ny); s <= s1; s++) hm[(size_t)s] = 1;
+      }
   }
   std::vector<int> slot(hm.size());
   int n = 0;
@@ -352,13 +364,14 @@ int wt_create(int nx, int ny, int nz, int storage, wt_lattice** out) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device);
     const int gx = (nx + wt::STEP_BX - 1) / wt::STEP_BX;
+    h->l2 = l2;
     const bool small = (double)n * 19 * elem_size(storage) <= 2.0 * (double)l2;
     h->pf = storage == WT_STORE_F16DEV && small ? (long long)sms * 8 * nx / gx / 3 : 0;
     if (const char* e = getenv("WT_PREFETCH_CELLS")) h->pf = std::max(0LL, atoll(e));
   }
-  h->nsegs = (long long)((nx + 31) / 32) * ny * nz;
+  h->nsegs = wt::segs_per_plane(nx, ny) * nz;
   const size_t pop = (size_t)n * 19 * h->elem;
-  if (const cudaError_t e = wt::configure_step_kernels(); e != cudaSuccess) {
+  if (const cudaError_t e = wt::configure_step_kernels(nx, storage); e != cudaSuccess) {
     cudaGetLastError();
     delete h;
     g_create_error = std::string("setting the step kernels' attributes failed: ") +
@@ -1088,7 +1101,7 @@ int adjoint_run(wt_lattice* h, const wt_adj_cfg& cfg, int C, double* dJds, wt_ad
   WT_CUDA(h, adj_done.make((size_t)ncp, cudaEventDisableTiming));
   cudaEvent_t e0 = ev.e[0], e1 = ev.e[1], e2 = ev.e[2];
   WT_CUDA(h, cudaMemsetAsync(h->err_dev, 0, sizeof(unsigned), h->stream));
-  const dim3 grid = wt::step_grid(h->nx, h->ny, h->nz);
+  const dim3 grid = wt::step_grid(make_args<S>(h));
   const bool wide = 19 * h->n >= (1LL << 31);
   WT_CUDA(h, cudaEventRecord(e0, h->stream));
   // forward sweep: a checkpoint every C steps, the force series for J

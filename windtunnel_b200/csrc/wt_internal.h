@@ -15,6 +15,7 @@ struct wt_lattice {
   int nx = 0, ny = 0, nz = 0, storage = 0;
   long long n = 0;
   int device = 0;
+  int l2 = 0;                    // L2 bytes of the device
   long long pf = 0;              // L2 prefetch distance of the lean kernel (cells)
   size_t elem = 4;               // bytes per stored population
   cudaStream_t stream = nullptr;
@@ -31,7 +32,7 @@ struct wt_lattice {
   float* uwy = nullptr;
   float* uwz = nullptr;
   // per-step force reduction: one partial per 32-cell segment holding a near-wall cell
-  long long nsegs = 0;           // 32-cell row segments of the lattice
+  long long nsegs = 0;           // 32-cell segments of the lattice (seg_of)
   int* wslot = nullptr;          // per segment: partial slot or -1
   int nslots = 0;                // segments with a slot
   int part_cap = 0;              // slots that fit in `part` (per step of a chunk)
@@ -96,7 +97,7 @@ void launch_pair_f32(const StepArgs<float>& a, dim3 grid, bool wide, cudaStream_
 
 // Launch attributes of the step kernels (the pair kernels' L1 carveout), set
 // once per lattice creation.
-cudaError_t configure_step_kernels();
+cudaError_t configure_step_kernels(int nx, int storage);
 
 // Load the device code of every step and reduction kernel a wt_step call can
 // launch (cudaFuncGetAttributes on each), so that none is loaded lazily

@@ -11,14 +11,21 @@
 
 namespace wt {
 
+template <class S>
+using StepKernel = void (*)(StepArgs<S>);
+
+template <class S>
+static StepKernel<S> exact_kernel(bool wide, bool mov) {
+  if (wide) return mov ? k_step<S, true, long long, true> : k_step<S, true, long long, false>;
+  return mov ? k_step<S, true, int, true> : k_step<S, true, int, false>;
+}
+
 void launch_step_f32_exact(const StepArgs<float>& a, dim3 grid, bool wide, cudaStream_t s) {
-  if (wide) launch_pdl(k_step<float, true, long long>, grid, dim3(STEP_BX), s, a);
-  else launch_pdl(k_step<float, true, int>, grid, dim3(STEP_BX), s, a);
+  launch_pdl(exact_kernel<float>(wide, a.mov != 0), grid, dim3(STEP_BX), s, a);
 }
 
 void launch_step_f64_exact(const StepArgs<double>& a, dim3 grid, bool wide, cudaStream_t s) {
-  if (wide) launch_pdl(k_step<double, true, long long>, grid, dim3(STEP_BX), s, a);
-  else launch_pdl(k_step<double, true, int>, grid, dim3(STEP_BX), s, a);
+  launch_pdl(exact_kernel<double>(wide, a.mov != 0), grid, dim3(STEP_BX), s, a);
 }
 
 void launch_pbb_f32_exact(const StepArgs<float>& a, dim3 grid, bool wide, cudaStream_t s) {
@@ -43,12 +50,13 @@ void launch_adj_f64(const StepArgs<double>& a, const double* Tn, double* Tc, dou
 
 cudaError_t preload_exact_step_kernels() {
   cudaFuncAttributes fa;
-  const void* fns[] = {(const void*)k_step<float, true, int>, (const void*)k_step<float, true, long long>,
-                       (const void*)k_step<double, true, int>,
-                       (const void*)k_step<double, true, long long>};
-  for (const void* f : fns) {
-    const cudaError_t e = cudaFuncGetAttributes(&fa, f);
-    if (e != cudaSuccess) return e;
+  for (int k = 0; k < 4; k++) {
+    const bool wide = k & 1, mov = k & 2;
+    for (const void* f : {(const void*)exact_kernel<float>(wide, mov),
+                          (const void*)exact_kernel<double>(wide, mov)}) {
+      const cudaError_t e = cudaFuncGetAttributes(&fa, f);
+      if (e != cudaSuccess) return e;
+    }
   }
   return cudaSuccess;
 }

@@ -9,13 +9,13 @@
 namespace wt {
 
 void launch_step_f32_fast(const StepArgs<float>& a, dim3 grid, bool wide, cudaStream_t s) {
-  if (wide) launch_pdl(k_step<float, false, long long>, grid, dim3(STEP_BX), s, a);
-  else launch_pdl(k_step<float, false, int>, grid, dim3(STEP_BX), s, a);
+  if (wide) launch_pdl(k_step<float, false, long long, true>, grid, dim3(STEP_BX), s, a);
+  else launch_pdl(k_step<float, false, int, true>, grid, dim3(STEP_BX), s, a);
 }
 
 void launch_step_f16_fast(const StepArgs<__half>& a, dim3 grid, bool wide, cudaStream_t s) {
-  if (wide) launch_pdl(k_step<__half, false, long long>, grid, dim3(STEP_BX), s, a);
-  else launch_pdl(k_step<__half, false, int>, grid, dim3(STEP_BX), s, a);
+  if (wide) launch_pdl(k_step<__half, false, long long, true>, grid, dim3(STEP_BX), s, a);
+  else launch_pdl(k_step<__half, false, int, true>, grid, dim3(STEP_BX), s, a);
 }
 
 void launch_lean_f32(const StepArgs<float>& a, dim3 grid, bool, cudaStream_t s) {
@@ -26,30 +26,71 @@ void launch_lean_f16(const StepArgs<__half>& a, dim3 grid, bool, cudaStream_t s)
   launch_pdl(k_step_lean<__half>, grid, dim3(STEP_BX), s, a);
 }
 
-template <class S>
-inline dim3 pair_grid(int nx, int ny, int nz) {
-  constexpr int seg = 2 * pair_bx<S>();   // cells per block
-  return dim3((unsigned)((nx + seg - 1) / seg), (unsigned)ny, (unsigned)nz);
-}
-
 // Every step kernel (direct, lean, pair, partial bounce-back, adjoint)
 // launches with programmatic dependent launch (launch_pdl): a step's blocks
 // fill the slots the previous step's tail frees and start the moment it
 // completes. Measured on B200: pair float32 +2.5% on 256x128x128, half
 // storage +1-2%; the partial-bounce-back step on 128x64x64 +10%.
+// The pair kernel's variant for a lattice, and the grid it runs on.
 template <class S>
-void launch_pair_pdl(void (*k)(StepArgs<S>), const StepArgs<S>& a, cudaStream_t s) {
-  launch_pdl(k, pair_grid<S>(a.nx, a.ny, a.nz), dim3(pair_bx<S>()), s, a);
+inline int pair_mode(const StepArgs<S>& a) {
+  const bool rows = a.nx % (2 * PAIR_BX) == 0 && !a.zfast;
+  return (a.nx % 2 ? PAIR_ODD : (rows ? PAIR_ROWS : 0)) | (a.mov ? PAIR_MOV : 0);
 }
 
-void launch_pair_f16(const StepArgs<__half>& a, dim3, bool, cudaStream_t s) {
-  if (a.f16_sr) launch_pair_pdl<__half>(k_step_pair<__half, true>, a, s);
-  else launch_pair_pdl<__half>(k_step_pair<__half, false>, a, s);
+template <class S>
+inline dim3 pair_grid(const StepArgs<S>& a, int mode) {
+  const long long per = 2 * PAIR_BX;   // cells per block
+  if (mode & PAIR_ROWS)
+    return dim3((unsigned)(a.nx / per), (unsigned)a.ny, (unsigned)a.nz);
+  const long long cells = (long long)row_cells(a.nx) * a.ny;
+  return plane_grid((cells + per - 1) / per, a.nz, a.zfast != 0);
 }
 
-void launch_pair_f32(const StepArgs<float>& a, dim3, bool, cudaStream_t s) {
-  launch_pair_pdl<float>(k_step_pair<float, false>, a, s);
+template <class S>
+using PairKernel = void (*)(StepArgs<S>);
+
+template <class S>
+PairKernel<S> pair_kernel(bool sr, int mode) {
+  if constexpr (sizeof(S) == 2) {
+    if (sr) return mode & PAIR_ROWS ? k_step_pair<S, true, PAIR_ROWS> : k_step_pair<S, true, 0>;
+    return mode & PAIR_ROWS ? k_step_pair<S, false, PAIR_ROWS> : k_step_pair<S, false, 0>;
+  } else {
+    switch (mode) {
+      case PAIR_ODD: return k_step_pair<S, false, PAIR_ODD>;
+      case PAIR_MOV: return k_step_pair<S, false, PAIR_MOV>;
+      case PAIR_ODD | PAIR_MOV: return k_step_pair<S, false, PAIR_ODD | PAIR_MOV>;
+      case PAIR_ROWS: return k_step_pair<S, false, PAIR_ROWS>;
+      case PAIR_ROWS | PAIR_MOV: return k_step_pair<S, false, PAIR_ROWS | PAIR_MOV>;
+      default: return k_step_pair<S, false, 0>;
+    }
+  }
 }
+
+// Every variant, for the preload loop below.
+constexpr int kPairModes[] = {0, PAIR_ROWS, PAIR_ODD, PAIR_MOV, PAIR_ROWS | PAIR_MOV,
+                              PAIR_ODD | PAIR_MOV};
+template <class F>
+cudaError_t each_pair_kernel(F f) {
+  cudaError_t e = cudaSuccess;
+  for (int m : kPairModes) {
+    if (e == cudaSuccess) e = f((const void*)pair_kernel<float>(false, m));
+    for (bool sr : {false, true})
+      if (e == cudaSuccess && !(m & (PAIR_ODD | PAIR_MOV)))
+        e = f((const void*)pair_kernel<__half>(sr, m));
+  }
+  return e;
+}
+
+template <class S>
+void launch_pair(const StepArgs<S>& a, cudaStream_t s) {
+  const int mode = pair_mode(a);
+  launch_pdl(pair_kernel<S>(a.f16_sr != 0, mode), pair_grid(a, mode), dim3(PAIR_BX), s, a);
+}
+
+void launch_pair_f16(const StepArgs<__half>& a, dim3, bool, cudaStream_t s) { launch_pair(a, s); }
+
+void launch_pair_f32(const StepArgs<float>& a, dim3, bool, cudaStream_t s) { launch_pair(a, s); }
 
 // ---- partial bounce-back and adjoint (float32 arithmetic) -------------------------
 
@@ -131,35 +172,40 @@ void launch_force_reduce(const double* part, unsigned nslots, int nsteps, double
   k_force_reduce<<<nsteps, RED_T, 0, s>>>(part, nslots, out);
 }
 
-cudaError_t configure_step_kernels() {
+cudaError_t configure_step_kernels(int nx, int storage) {
   // The pair kernels use no shared memory: the whole unified L1 / shared
   // array goes to L1 (measured on B200: +1.6% for half storage on
-  // 256x128x128, +0.5% on 512x192x192, float32 unchanged).
-  const void* fns[] = {(const void*)k_step_pair<__half, false>,
-                       (const void*)k_step_pair<__half, true>,
-                       (const void*)k_step_pair<float, false>};
-  for (const void* f : fns) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
-    if (e != cudaSuccess) return e;
+  // 256x128x128, +0.5% on 512x192x192, float32 unchanged). Only the variants a
+  // lattice of this width can launch are touched.
+  auto l1 = [](auto* f) {
+    return cudaFuncSetAttribute((const void*)f, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
+  };
+  const int m = nx % 2 ? PAIR_ODD : (nx % (2 * PAIR_BX) == 0 ? PAIR_ROWS : 0);
+  cudaError_t e = cudaSuccess;
+  if (storage == WT_STORE_F32) {
+    e = l1(pair_kernel<float>(false, m));
+    if (e == cudaSuccess) e = l1(pair_kernel<float>(false, m | PAIR_MOV));
+  } else if (storage == WT_STORE_F16DEV && !(m & PAIR_ODD)) {
+    e = l1(pair_kernel<__half>(false, m));
+    if (e == cudaSuccess) e = l1(pair_kernel<__half>(true, m));
   }
-  return cudaSuccess;
+  return e;
 }
 
 cudaError_t preload_step_kernels() {
   cudaFuncAttributes fa;
   const void* fns[] = {
-      (const void*)k_step<float, false, int>, (const void*)k_step<float, false, long long>,
-      (const void*)k_step<__half, false, int>, (const void*)k_step<__half, false, long long>,
+      (const void*)k_step<float, false, int, true>, (const void*)k_step<float, false, long long, true>,
+      (const void*)k_step<__half, false, int, true>, (const void*)k_step<__half, false, long long, true>,
       (const void*)k_step_lean<float>, (const void*)k_step_lean<__half>,
-      (const void*)k_step_pair<__half, false>, (const void*)k_step_pair<__half, true>,
-      (const void*)k_step_pair<float, false>,
       (const void*)k_force_reduce};
   for (const void* f : fns) {
     const cudaError_t e = cudaFuncGetAttributes(&fa, f);
     if (e != cudaSuccess) return e;
   }
-  return preload_exact_step_kernels();
+  const cudaError_t e =
+      each_pair_kernel([&](const void* f) { return cudaFuncGetAttributes(&fa, f); });
+  return e != cudaSuccess ? e : preload_exact_step_kernels();
 }
 
 }  // namespace wt

@@ -351,16 +351,18 @@ template <class S, bool EXACT, class IDX>
 __global__ void __launch_bounds__(STEP_BX) k_step_pbb(const __grid_constant__ StepArgs<S> a) {
   using M = typename std::conditional<EXACT, double, float>::type;
   pdl_enter();
-  const int x = blockIdx.x * STEP_BX + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
+  const Cell3 cell = step_cell(a);
+  const int x = cell.x, y = cell.y, z = cell.z;
   const long long i = (long long)x + (long long)a.nx * y + a.nxy * z;
   double Fx = 0, Fy = 0, Fz = 0;
   // Every 32-cell segment that touches the box owns a force slot and must
   // write it every step (zeros where nothing is exchanged): cells of the box
   // take part in the warp's partial whatever their category.
-  bool near_cell = x < a.nx && x >= a.sb[0] && x < a.sb[3] && y >= a.sb[1] && y < a.sb[4] &&
-                   z >= a.sb[2] && z < a.sb[5];
-  if (x < a.nx - 1) {
+  // An outlet cell without a thread of its own (odd nx) belongs to cell nx-2's.
+  const bool last = x == row_cells(a.nx) - 1;
+  bool near_cell = x < a.sb[3] && (last ? a.nx - 1 : x) >= a.sb[0] && y >= a.sb[1] &&
+                   y < a.sb[4] && z >= a.sb[2] && z < a.sb[5];
+  if (x < a.nx - 1 && y < a.ny) {
     int cat;
     uint8_t fl = 0;
     const bool dup = (x == a.nx - 2);
@@ -378,11 +380,17 @@ __global__ void __launch_bounds__(STEP_BX) k_step_pbb(const __grid_constant__ St
       CellFw<M> c;
       const bool wall = (fl & FLAG_NEAR) != 0;
       near_cell = near_cell || wall;
-      const bool shell = a.freeslip && (y == 1 || y == a.ny - 2 || z == 1 || z == a.nz - 2);
       const S* Fi = a.F + i;
+      const ShellRow row = shell_row(a, y, z);
+      if (!row.any()) {
 #pragma unroll
-      for (int q = 0; q < Q; q++) c.f[q] = ld<M>(Fi[(IDX)a.src[q]]);
-      if (wall || shell) patch_special<S, M>(a, i, x, y, z, shell, c.f, Fx, Fy, Fz);
+        for (int q = 0; q < Q; q++) c.f[q] = ld<M>(Fi[(IDX)a.src[q]]);
+      } else {
+#define WT_PULL(q) c.f[q] = ld<M>(Fi[(IDX)shell_src<q>(a, row)]);
+        WT_EACH_Q(WT_PULL)
+#undef WT_PULL
+      }
+      if (wall) patch_bounce<S, M, M, true>(a, i, c.f, Fx, Fy, Fz);
       cell_fw<M>(a, c);
       if (!(c.r > (M)0 && c.r < (M)1.0e30)) atomicOr(a.err, 1u);
       if (a.write_fields) {
@@ -427,8 +435,11 @@ __global__ void __launch_bounds__(STEP_BX) k_step_pbb(const __grid_constant__ St
         if (dup) { a.ux[i + 1] = a.u0f; a.uy[i + 1] = 0.0f; a.uz[i + 1] = 0.0f; a.rho[i + 1] = 1.0f; }
       }
     } else if (dup) {
+      S v[Q];
 #pragma unroll
-      for (int q = 0; q < Q; q++) Gi[(IDX)a.dst[q] + 1] = Gi[(IDX)a.dst[q]];
+      for (int q = 0; q < Q; q++) v[q] = Gi[(IDX)a.dst[q]];
+#pragma unroll
+      for (int q = 0; q < Q; q++) Gi[(IDX)a.dst[q] + 1] = v[q];
       if (a.write_fields) {
         a.ux[i + 1] = a.ux[i]; a.uy[i + 1] = a.uy[i]; a.uz[i + 1] = a.uz[i]; a.rho[i + 1] = a.rho[i];
       }
@@ -449,6 +460,7 @@ struct AdjArgs {
   long long gat[Q];   // element offset from cell i to its link-q consumer: q*n + ex + nx ey + nxy ez
   uint32_t gatb[Q];   // gat[q] * sizeof(T) (non-negative), when every offset fits in 31 bits
   uint32_t rowb[Q];   // q*n * sizeof(T), likewise
+  FastDiv col;        // nx: index of a cell in its plane -> y
 };
 
 // The free-slip term of the adjoint of the population stored at (q, location
@@ -498,10 +510,10 @@ template <class S, class T, bool NB>
 __global__ void __launch_bounds__(STEP_BX, adj_min_blocks<S, T>()) k_adjoint(const __grid_constant__ StepArgs<S> a,
                                                          const __grid_constant__ AdjArgs<T> j) {
   pdl_enter();
-  const int x = blockIdx.x * STEP_BX + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
-  const long long i = (long long)x + (long long)a.nx * y + a.nxy * z;
-  if (x >= a.nx) return;
+  const unsigned p = blockIdx.x * STEP_BX + threadIdx.x;
+  if (p >= (unsigned)a.nxy) return;
+  const int y = (int)j.col.div(p), x = (int)(p - (unsigned)y * j.col.d), z = blockIdx.y;
+  const long long i = (long long)p + a.nxy * z;
   const bool inner = x >= 1 && x <= a.nx - 2 && y >= 1 && y <= a.ny - 2 && z >= 1 &&
                      z <= a.nz - 2;
   T* Tci = j.Tc + i;
@@ -660,7 +672,8 @@ inline void launch_adjoint(const StepArgs<S>& a, const T* Tn, T* Tc, double* ds,
     j.gatb[q] = nb ? (uint32_t)(j.gat[q] * (long long)sizeof(T)) : 0u;
     j.rowb[q] = nb ? (uint32_t)(q * a.n * (long long)sizeof(T)) : 0u;
   }
-  const dim3 grid = step_grid(a.nx, a.ny, a.nz);
+  j.col = fast_div((unsigned)a.nx);
+  const dim3 grid((unsigned)((a.nxy + STEP_BX - 1) / STEP_BX), (unsigned)a.nz);
   if (nb) launch_pdl(k_adjoint<S, T, true>, grid, dim3(STEP_BX), s, a, j);
   else launch_pdl(k_adjoint<S, T, false>, grid, dim3(STEP_BX), s, a, j);
 }

@@ -77,64 +77,105 @@ __device__ __forceinline__ void warp_force_partial_w(double fx, double fy, doubl
   }
 }
 
-// Warp partial of the direct kernel: its warps cover 32-cell segments.
+// Warp partial of the one-cell-per-thread kernels: their warps cover 32-cell
+// segments.
 template <class S>
 __device__ __forceinline__ void warp_force_partial(double fx, double fy, double fz,
                                                    bool near_cell, const StepArgs<S>& a) {
-  const int x0 = blockIdx.x * STEP_BX + (threadIdx.x & ~31);
-  warp_force_partial_w(fx, fy, fz, near_cell, a, seg_of(x0, blockIdx.y, blockIdx.z, a.nx, a.ny));
+  const long long seg = plane_of(a) * segs_per_plane(a.nx, a.ny) +
+                        (long long)block_of(a) * (STEP_BX / 32) + (threadIdx.x >> 5);
+  warp_force_partial_w(fx, fy, fz, near_cell, a, seg);
 }
 
-// Bounce-back link q of cell i toward solid neighbour j (code s):
-// js/lbm.js:339-359. Returns the pulled population and accumulates the
-// momentum exchange of links into the body (SOLID_OBJ).
-template <class S, class M, int q>
-__device__ __forceinline__ M bounce_link(const StepArgs<S>& a, long long i, long long j, int s,
-                                         M rho_prev, double& Fx, double& Fy, double& Fz) {
-  const M fd = ld<M>(a.F[opp(q) * a.n + i]);
-  M corr = 0;
-  if (a.mov) {
-    const M cu = (M)ex(q) * (M)a.uwx[j] + (M)ey(q) * (M)a.uwy[j] + (M)ez(q) * (M)a.uwz[j];
-    if (cu != (M)0) corr = (M)6 * (M)wq(q) * rho_prev * cu;
-  }
-  if (s == WT_SOLID_OBJ) {
-    const M d = (M)2 * fd + corr;
-    Fx -= (double)(d * (M)ex(q));
-    Fy -= (double)(d * (M)ey(q));
-    Fz -= (double)(d * (M)ez(q));
-  }
-  return fd + corr;
+// Free-slip side planes: a cell of the layer beside one (y = 1 or ny-2, z = 1
+// or nz-2) pulls a direction whose source lies on the plane as the mirrored
+// direction of the source reflected into the layer itself, same x - ex. Which
+// directions those are depends on the row alone, so a shell row's loads take
+// the mirrored offset at once instead of overwriting plain values afterwards
+// (one memory latency instead of two, which the last planes of a step have
+// nothing to hide behind; B200, 256x128x128 float32, free-slip against equilibrium
+// sides: 98.9 against 96.3 us a step with overwriting, 96.5 against 96.4 so).
+struct ShellRow {
+  bool y1, yn, z1, zn;
+  __device__ __forceinline__ bool any() const { return y1 || yn || z1 || zn; }
+};
+
+template <class S>
+__device__ __forceinline__ ShellRow shell_row(const StepArgs<S>& a, int y, int z) {
+  const bool fs = a.freeslip != 0;
+  return ShellRow{fs && y == 1, fs && y == a.ny - 2, fs && z == 1, fs && z == a.nz - 2};
 }
+
+// Element offset, from a shell cell, of the value its direction q pulls.
+template <int q, class S>
+__device__ __forceinline__ long long shell_src(const StepArgs<S>& a, const ShellRow& r) {
+  if constexpr (ey(q) == 0 && ez(q) == 0) return a.src[q];
+  const bool ym = ey(q) == 1 ? r.y1 : (ey(q) == -1 ? r.yn : false);
+  const bool zm = ez(q) == 1 ? r.z1 : (ez(q) == -1 ? r.zn : false);
+  if (ym && zm) return mirror_z(mirror_y(q)) * a.n - ex(q);
+  if (ym) return mirror_y(q) * a.n - ex(q) - (long long)ez(q) * a.nxy;
+  if (zm) return mirror_z(q) * a.n - ex(q) - (long long)ey(q) * a.nx;
+  return a.src[q];
+}
+
+// X(q) for every direction.
+#define WT_EACH_Q(X)                                                                        \
+  X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) \
+  X(17) X(18)
 
 // Overwrite, in f (already holding the plain pulled values), the directions
-// whose source is solid (bounce-back) or lies on a free-slip side plane
-// (mirror gather). The solid / body neighbours come from the cell's
-// precomputed mask (one load); the loads below depend only on it and on the
-// cell position, so they are all in flight at once.
-template <class S, class M>
-__device__ __forceinline__ void patch_special(const StepArgs<S>& a, long long i, int x, int y,
-                                              int z, bool shell, M (&f)[Q], double& Fx,
-                                              double& Fy, double& Fz) {
+// whose source is solid (bounce-back, js/lbm.js:339-359), and accumulate the
+// momentum exchange of links into the body (SOLID_OBJ). The solid / body neighbours come from
+// the cell's precomputed mask (one load). Two passes: the first issues every
+// load of the cell (they depend only on the mask and the cell's position) and
+// consumes none, so that a near-wall warp waits for one memory latency
+// instead of one per link; the second forms corrections and forces (measured
+// on the pair kernel, pair_patch).
+// T: the type of the held values (S itself where it holds every pulled value
+// exactly, else the arithmetic type M); MOV as false drops the moving-wall
+// correction at compile time.
+template <class S, class M, class T, bool MOV>
+__device__ __forceinline__ void patch_bounce(const StepArgs<S>& a, long long i, T (&f)[Q],
+                                             double& Fx, double& Fy, double& Fz) {
   const unsigned long long m = a.nmask[i];
   const unsigned sm = (unsigned)m, om = (unsigned)(m >> 32);
-  const M rho_prev = (M)(a.mov && sm ? a.rho[i] : 1.0f);
+  const bool mov = MOV && a.mov && sm;
+  const M rho_prev = (M)(mov ? a.rho[i] : 1.0f);
+  M cu[MOV ? Q : 1];
+  auto held = [](S v) -> T {
+    if constexpr (std::is_same<T, S>::value) return v;
+    else return ld<T>(v);
+  };
 #define WT_PATCH(q)                                                                         \
+  if constexpr (MOV) cu[q] = (M)0;                                                          \
   if ((sm >> (q)) & 1u) {                                                                   \
-    const long long j = i - (ex(q) + (long long)ey(q) * a.nx + (long long)ez(q) * a.nxy);   \
-    f[q] = bounce_link<S, M, q>(a, i, j, ((om >> (q)) & 1u) ? WT_SOLID_OBJ : WT_SOLID_WALL, \
-                                rho_prev, Fx, Fy, Fz);                                      \
-  } else if (shell) {                                                                       \
-    int sy = y - ey(q), sz = z - ez(q), qq = q;                                             \
-    bool refl = false;                                                                      \
-    if (sy == 0 || sy == a.ny - 1) { sy = y; qq = mirror_y(qq); refl = true; }              \
-    if (sz == 0 || sz == a.nz - 1) { sz = z; qq = mirror_z(qq); refl = true; }              \
-    if (refl)                                                                               \
-      f[q] = ld<M>(a.F[qq * a.n + (x - ex(q)) + (long long)a.nx * sy + a.nxy * sz]);        \
+    f[q] = held(a.F[opp(q) * a.n + i]);                                                     \
+    if (MOV && mov) {                                                                       \
+      const long long j = i - (ex(q) + (long long)ey(q) * a.nx + (long long)ez(q) * a.nxy); \
+      cu[q] = (M)ex(q) * (M)a.uwx[j] + (M)ey(q) * (M)a.uwy[j] + (M)ez(q) * (M)a.uwz[j];     \
+    }                                                                                       \
   }
-  WT_PATCH(1) WT_PATCH(2) WT_PATCH(3) WT_PATCH(4) WT_PATCH(5) WT_PATCH(6) WT_PATCH(7)
-  WT_PATCH(8) WT_PATCH(9) WT_PATCH(10) WT_PATCH(11) WT_PATCH(12) WT_PATCH(13) WT_PATCH(14)
-  WT_PATCH(15) WT_PATCH(16) WT_PATCH(17) WT_PATCH(18)
+  WT_EACH_Q(WT_PATCH)
 #undef WT_PATCH
+  if (!(om || mov)) return;
+#define WT_LINK(q)                                                             \
+  if (((MOV && mov ? sm : om) >> (q)) & 1u) {                                  \
+    M fd, corr = (M)0;                                                         \
+    if constexpr (std::is_same<T, S>::value) fd = ld<M>(f[q]);                 \
+    else fd = f[q];                                                            \
+    if constexpr (MOV) {                                                       \
+      if (cu[q] != (M)0) corr = (M)6 * (M)wq(q) * rho_prev * cu[q];            \
+      if constexpr (std::is_same<T, M>::value) f[q] = fd + corr;               \
+    }                                                                          \
+    if ((om >> (q)) & 1u) {                                                    \
+      const M d = (M)2 * fd + corr;                                            \
+      Fx -= (double)(d * (M)ex(q));                                            \
+      Fy -= (double)(d * (M)ey(q));                                            \
+      Fz -= (double)(d * (M)ez(q));                                            \
+    }                                                                          \
+  }
+  WT_EACH_Q(WT_LINK)
+#undef WT_LINK
 }
 
 // Hardware approximations (relative error ~2^-22) used by the float32
@@ -261,21 +302,36 @@ __device__ __forceinline__ void collide_fast(const StepArgs<S>& a, const float (
 // translation unit that instantiates it is compiled with --fmad=false, so no
 // multiply-add is contracted and every rounding matches the reference's
 // IEEE double arithmetic; results are rounded to S only at the stores.
-template <class S, class Out>
-__device__ __forceinline__ void collide_exact(const StepArgs<S>& a, const double (&fq)[Q],
-                                              long long i, bool dup, bool near_cell, Out out) {
-  const double f0 = fq[0], f1 = fq[1], f2 = fq[2], f3 = fq[3], f4 = fq[4], f5 = fq[5],
-               f6 = fq[6], f7 = fq[7], f8 = fq[8], f9 = fq[9], f10 = fq[10], f11 = fq[11],
-               f12 = fq[12], f13 = fq[13], f14 = fq[14], f15 = fq[15], f16 = fq[16],
-               f17 = fq[17], f18 = fq[18];
-  const double dr = f0 + f1 + f2 + f3 + f4 + f5 + f6 + f7 + f8 + f9 + f10 + f11 + f12 + f13 +
-                    f14 + f15 + f16 + f17 + f18;
-  const double r = 1 + dr;
-  if (!(r > 0.0 && r < 1.0e300)) atomicOr(a.err, 1u);
-  const double inv = 1 / r;
-  const double vx = (f1 - f2 + f7 - f8 + f9 - f10 + f11 - f12 + f13 - f14) * inv;
-  const double vy = (f3 - f4 + f7 - f8 - f9 + f10 + f15 - f16 + f17 - f18) * inv;
-  const double vz = (f5 - f6 + f11 - f12 - f13 + f14 + f15 - f16 - f17 + f18) * inv;
+// Two passes over the populations, which are held as T (the storage type
+// where it represents them exactly): the first adds each non-equilibrium part
+// n_q = f_q - e_q into the stress sums as soon as it is formed (the sums of
+// js/lbm.js:420-425 run in ascending q, so their order is kept), the second
+// forms e_q and n_q again and writes each output pair. The 18 doubles n_q are
+// then never live together: 30% more float64 operations for half the
+// registers. `opaque` keeps the compiler from merging the passes again.
+__device__ __forceinline__ void opaque(double& v) { asm volatile("" : "+d"(v)); }
+__device__ __forceinline__ void opaque(float& v) { asm volatile("" : "+f"(v)); }
+
+template <class S, class T, class Out>
+__device__ __forceinline__ void collide_exact(const StepArgs<S>& a, T (&f)[Q], long long i,
+                                              bool dup, bool near_cell, Out out) {
+  constexpr double W0 = 1.0 / 3, WF = 1.0 / 18, WE = 1.0 / 36;
+  auto fd = [&](int q) -> double { return (double)f[q]; };
+  double dr, vx, vy, vz, r, inv;
+  {
+    const double f0 = fd(0), f1 = fd(1), f2 = fd(2), f3 = fd(3), f4 = fd(4), f5 = fd(5),
+                 f6 = fd(6), f7 = fd(7), f8 = fd(8), f9 = fd(9), f10 = fd(10), f11 = fd(11),
+                 f12 = fd(12), f13 = fd(13), f14 = fd(14), f15 = fd(15), f16 = fd(16),
+                 f17 = fd(17), f18 = fd(18);
+    dr = f0 + f1 + f2 + f3 + f4 + f5 + f6 + f7 + f8 + f9 + f10 + f11 + f12 + f13 + f14 + f15 +
+         f16 + f17 + f18;
+    r = 1 + dr;
+    if (!(r > 0.0 && r < 1.0e300)) atomicOr(a.err, 1u);
+    inv = 1 / r;
+    vx = (f1 - f2 + f7 - f8 + f9 - f10 + f11 - f12 + f13 - f14) * inv;
+    vy = (f3 - f4 + f7 - f8 - f9 + f10 + f15 - f16 + f17 - f18) * inv;
+    vz = (f5 - f6 + f11 - f12 - f13 + f14 + f15 - f16 - f17 + f18) * inv;
+  }
   if (a.write_fields) {
     const float rf = __double2float_rn(r), xf = __double2float_rn(vx),
                 yf = __double2float_rn(vy), zf = __double2float_rn(vz);
@@ -284,116 +340,150 @@ __device__ __forceinline__ void collide_exact(const StepArgs<S>& a, const double
   } else if (a.mov && near_cell) {
     a.rho[i] = __double2float_rn(r);
   }
-  const double A = dr - r * 1.5 * (vx * vx + vy * vy + vz * vz);
-  const double r3 = 3 * r, r45 = 4.5 * r;
-  const double ax = vx, ay = vy, az = vz;
-  const double bxy = vx + vy, bxY = vx - vy;
-  const double bxz = vx + vz, bxZ = vx - vz;
-  const double byz = vy + vz, byZ = vy - vz;
-  constexpr double W0 = 1.0 / 3, WF = 1.0 / 18, WE = 1.0 / 36;
-  const double e0 = W0 * A;
-  const double hx = r45 * ax * ax, hy = r45 * ay * ay, hz = r45 * az * az;
-  const double e1 = WF * (A + r3 * ax + hx), e2 = WF * (A - r3 * ax + hx);
-  const double e3 = WF * (A + r3 * ay + hy), e4 = WF * (A - r3 * ay + hy);
-  const double e5 = WF * (A + r3 * az + hz), e6 = WF * (A - r3 * az + hz);
-  const double h7 = r45 * bxy * bxy, h9 = r45 * bxY * bxY;
-  const double h11 = r45 * bxz * bxz, h13 = r45 * bxZ * bxZ;
-  const double h15 = r45 * byz * byz, h17 = r45 * byZ * byZ;
-  const double e7 = WE * (A + r3 * bxy + h7), e8 = WE * (A - r3 * bxy + h7);
-  const double e9 = WE * (A + r3 * bxY + h9), e10 = WE * (A - r3 * bxY + h9);
-  const double e11 = WE * (A + r3 * bxz + h11), e12 = WE * (A - r3 * bxz + h11);
-  const double e13 = WE * (A + r3 * bxZ + h13), e14 = WE * (A - r3 * bxZ + h13);
-  const double e15 = WE * (A + r3 * byz + h15), e16 = WE * (A - r3 * byz + h15);
-  const double e17 = WE * (A + r3 * byZ + h17), e18 = WE * (A - r3 * byZ + h17);
-  const double n1 = f1 - e1, n2 = f2 - e2, n3 = f3 - e3, n4 = f4 - e4;
-  const double n5 = f5 - e5, n6 = f6 - e6, n7 = f7 - e7, n8 = f8 - e8;
-  const double n9 = f9 - e9, n10 = f10 - e10, n11 = f11 - e11, n12 = f12 - e12;
-  const double n13 = f13 - e13, n14 = f14 - e14, n15 = f15 - e15, n16 = f16 - e16;
-  const double n17 = f17 - e17, n18 = f18 - e18;
+  double A = dr - r * 1.5 * (vx * vx + vy * vy + vz * vz);
+  double r3 = 3 * r, r45 = 4.5 * r;
+  // equilibria of the opposite pair (k, k+1) along b = c_k . u, weight W:
+  // e_k = W (A + r3 b + h), e_{k+1} = W (A - r3 b + h), h = r45 b b
+#define WT_XEQ(W, B)                                     \
+  const double b_ = B, t_ = r3 * b_, h_ = r45 * b_ * b_; \
+  const double ea = W * (A + t_ + h_), eb = W * (A - t_ + h_);
   const double tau0 = a.tau0;
   double om = a.omega0, tauEff = tau0;
   if (a.les) {
-    const double pxx = n1 + n2 + n7 + n8 + n9 + n10 + n11 + n12 + n13 + n14;
-    const double pyy = n3 + n4 + n7 + n8 + n9 + n10 + n15 + n16 + n17 + n18;
-    const double pzz = n5 + n6 + n11 + n12 + n13 + n14 + n15 + n16 + n17 + n18;
-    const double pxy = n7 + n8 - n9 - n10;
-    const double pxz = n11 + n12 - n13 - n14;
-    const double pyz = n15 + n16 - n17 - n18;
+    double pxx, pyy, pzz, pxy, pxz, pyz;
+#define WT_XN(k, W, B) WT_XEQ(W, B) const double na = fd(k) - ea, nb = fd(k + 1) - eb;
+    { WT_XN(1, WF, vx) pxx = na + nb; }
+    { WT_XN(3, WF, vy) pyy = na + nb; }
+    { WT_XN(5, WF, vz) pzz = na + nb; }
+    { WT_XN(7, WE, vx + vy) pxx = pxx + na + nb; pyy = pyy + na + nb; pxy = na + nb; }
+    { WT_XN(9, WE, vx - vy) pxx = pxx + na + nb; pyy = pyy + na + nb; pxy = pxy - na - nb; }
+    { WT_XN(11, WE, vx + vz) pxx = pxx + na + nb; pzz = pzz + na + nb; pxz = na + nb; }
+    { WT_XN(13, WE, vx - vz) pxx = pxx + na + nb; pzz = pzz + na + nb; pxz = pxz - na - nb; }
+    { WT_XN(15, WE, vy + vz) pyy = pyy + na + nb; pzz = pzz + na + nb; pyz = na + nb; }
+    { WT_XN(17, WE, vy - vz) pyy = pyy + na + nb; pzz = pzz + na + nb; pyz = pyz - na - nb; }
+#undef WT_XN
     const double mag = sqrt(2 * (pxx * pxx + pyy * pyy + pzz * pzz +
                                  2 * (pxy * pxy + pxz * pxz + pyz * pyz)));
     const double SQ18 = 18 * 1.4142135623730951;
     tauEff = 0.5 * (tau0 + sqrt(tau0 * tau0 + SQ18 * a.cs2 * mag * inv));
     om = 1 / tauEff;
+    opaque(A); opaque(r3); opaque(r45); opaque(vx); opaque(vy); opaque(vz);
+    if constexpr (!std::is_same<T, double>::value) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) opaque(f[q]);
+    }
   }
   const double omm = a.trt ? 1 / (0.5 + a.lam / (tauEff - 0.5)) : om;
-  out.put(0, Store<S>::from_d(f0 - om * (f0 - e0)));
-  double sp, sm;
-#define WT_XOUT(A_, B_, NA, NB, FA, FB)                   \
-  sp = 0.5 * (NA + NB); sm = 0.5 * (NA - NB);             \
-  out.put(A_, Store<S>::from_d(FA - om * sp - omm * sm)); \
-  out.put(B_, Store<S>::from_d(FB - om * sp + omm * sm));
-  WT_XOUT(1, 2, n1, n2, f1, f2)
-  WT_XOUT(3, 4, n3, n4, f3, f4)
-  WT_XOUT(5, 6, n5, n6, f5, f6)
-  WT_XOUT(7, 8, n7, n8, f7, f8)
-  WT_XOUT(9, 10, n9, n10, f9, f10)
-  WT_XOUT(11, 12, n11, n12, f11, f12)
-  WT_XOUT(13, 14, n13, n14, f13, f14)
-  WT_XOUT(15, 16, n15, n16, f15, f16)
-  WT_XOUT(17, 18, n17, n18, f17, f18)
+  {
+    const double f0 = fd(0), e0 = W0 * A;
+    out.put(0, Store<S>::from_d(f0 - om * (f0 - e0)));
+  }
+#define WT_XOUT(k, W, B)                                      \
+  {                                                           \
+    WT_XEQ(W, B)                                              \
+    const double fa = fd(k), fb = fd(k + 1);                  \
+    const double na = fa - ea, nb = fb - eb;                  \
+    const double sp = 0.5 * (na + nb), sm = 0.5 * (na - nb);  \
+    out.put(k, Store<S>::from_d(fa - om * sp - omm * sm));    \
+    out.put(k + 1, Store<S>::from_d(fb - om * sp + omm * sm)); \
+  }
+  WT_XOUT(1, WF, vx)
+  WT_XOUT(3, WF, vy)
+  WT_XOUT(5, WF, vz)
+  WT_XOUT(7, WE, vx + vy)
+  WT_XOUT(9, WE, vx - vy)
+  WT_XOUT(11, WE, vx + vz)
+  WT_XOUT(13, WE, vx - vz)
+  WT_XOUT(15, WE, vy + vz)
+  WT_XOUT(17, WE, vy - vz)
 #undef WT_XOUT
+#undef WT_XEQ
 }
 
-// The float32 step is capped at 64 registers so that 8 blocks of 128 threads
-// stay resident per SM: the step is bound by memory latency, and resident
-// warps are what keep enough of the 19 load streams in flight. The float64
-// (exact) step keeps 128 registers rather than spill.
-constexpr int step_min_blocks(bool exact) { return exact ? 4 : 8; }
+// Output writer that stores straight to the cell (and, for the thread of
+// column nx-2, to the outlet cell beside it).
+template <class S, class IDX>
+struct CellOut {
+  S* g;
+  const StepArgs<S>& a;
+  bool dup;
+  __device__ __forceinline__ void put(int q, S v) const {
+    g[(IDX)a.dst[q]] = v;
+    if (dup) g[(IDX)a.dst[q] + 1] = v;
+  }
+};
+
+// Resident blocks per SM the register budget is set for. The float32 step is
+// capped at 64 registers so that 8 blocks of 128 threads stay resident per SM:
+// it is bound by memory latency, and resident warps are what keep enough of
+// the 19 load streams in flight. Exact step, measured on B200 (blocks:
+// microseconds a step): float64 storage, 192x96x96: 4: 93.9, 5: 85.8, 6: 83.9;
+// float32 storage, 96x44x44: 4: 11.3, 5: 10.4, 6: 10.8, 7: 11.3; with moving
+// walls the held values are doubles and 4 blocks leave them in registers.
+template <class S, bool EXACT, bool MOV>
+constexpr int step_min_blocks() {
+  return EXACT ? (MOV ? 4 : (sizeof(S) == 8 ? 6 : 5)) : 8;
+}
 
 // IDX is the type of the per-direction offsets: int when 19*n fits in 31
 // bits (every practical lattice), long long otherwise.
-template <class S, bool EXACT, class IDX>
-__global__ void __launch_bounds__(STEP_BX, step_min_blocks(EXACT)) k_step(const __grid_constant__ StepArgs<S> a) {
+template <class S, bool EXACT, class IDX, bool MOV>
+__global__ void __launch_bounds__(STEP_BX, step_min_blocks<S, EXACT, MOV>()) k_step(const __grid_constant__ StepArgs<S> a) {
   using M = typename std::conditional<EXACT, double, float>::type;
-  pdl_enter();   // programmatic dependent launch (launch_pdl)
-  const int x = blockIdx.x * STEP_BX + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
+  // held values: the storage type unless a moving-wall correction can leave it
+  using T = typename std::conditional<EXACT && !MOV, S, M>::type;
+  const Cell3 cell = step_cell(a);
+  const int x = cell.x, y = cell.y, z = cell.z;
   const long long i = (long long)x + (long long)a.nx * y + a.nxy * z;
   double Fx = 0, Fy = 0, Fz = 0;
   bool near_cell = false;
-  if (x < a.nx - 1) {
-    int cat;
-    uint8_t fl = 0;
-    const bool dup = (x == a.nx - 2);   // this thread also writes the outlet cell x+1
-    if (x == 0) {
-      cat = CAT_EQ;
-    } else {
-      fl = a.flags[i];
-      if (z == 0 || z == a.nz - 1 || y == a.ny - 1) cat = CAT_EQ;
-      else if (fl & FLAG_SOLID_MASK) cat = CAT_KEEP;
-      else if (y == 0) cat = CAT_EQ;
-      else cat = CAT_FLUID;
-    }
-    S* Gi = a.G + i;
-    if (cat == CAT_FLUID) {
-      M f[Q];
-      near_cell = (fl & FLAG_NEAR) != 0;
-      const bool shell = a.freeslip && (y == 1 || y == a.ny - 2 || z == 1 || z == a.nz - 2);
+  const bool inside = x < a.nx - 1 && y < a.ny;
+  const bool inner = inside && x > 0 && y > 0 && y < a.ny - 1 && z > 0 && z < a.nz - 1;
+  pdl_enter();   // programmatic dependent launch (launch_pdl)
+  if (inside) {
+    T f[Q];
+    // the pulls of every cell that can be fluid are issued before its flags
+    // byte is looked at: all their sources lie inside the lattice
+    if (inner) {
       const S* Fi = a.F + i;
+      auto held = [](S v) -> T {
+        if constexpr (std::is_same<T, S>::value) return v;
+        else return ld<T>(v);
+      };
+      const ShellRow row = shell_row(a, y, z);
+      if (!row.any()) {
 #pragma unroll
-      for (int q = 0; q < Q; q++) f[q] = ld<M>(Fi[(IDX)a.src[q]]);
-      if (near_cell || shell) patch_special<S, M>(a, i, x, y, z, shell, f, Fx, Fy, Fz);
-      S out[Q];
-      if constexpr (EXACT) {
-        collide_exact<S>(a, f, i, dup, near_cell, RegOut<S>{out});
+        for (int q = 0; q < Q; q++) f[q] = held(Fi[(IDX)a.src[q]]);
       } else {
-        collide_fast<S>(a, f, i, dup, near_cell, RegOut<S>{out});
+#define WT_PULL(q) f[q] = held(Fi[(IDX)shell_src<q>(a, row)]);
+        WT_EACH_Q(WT_PULL)
+#undef WT_PULL
       }
+    }
+    uint8_t fl = 0;
+    if (x > 0) fl = a.flags[i];
+    int cat;
+    const bool dup = (x == a.nx - 2);   // this thread also writes the outlet cell x+1
+    if (x == 0) cat = CAT_EQ;
+    else if (z == 0 || z == a.nz - 1 || y == a.ny - 1) cat = CAT_EQ;
+    else if (fl & FLAG_SOLID_MASK) cat = CAT_KEEP;
+    else if (y == 0) cat = CAT_EQ;
+    else cat = CAT_FLUID;
+    S* Gi = a.G + i;
+    if (cat == CAT_FLUID) {   // implies inner
+      near_cell = (fl & FLAG_NEAR) != 0;
+      if (near_cell) patch_bounce<S, M, T, MOV>(a, i, f, Fx, Fy, Fz);
+      if constexpr (EXACT) {
+        collide_exact<S>(a, f, i, dup, near_cell, CellOut<S, IDX>{Gi, a, dup});
+      } else {
+        S out[Q];
+        collide_fast<S>(a, f, i, dup, near_cell, RegOut<S>{out});
 #pragma unroll
-      for (int q = 0; q < Q; q++) Gi[(IDX)a.dst[q]] = out[q];
-      if (dup) {
+        for (int q = 0; q < Q; q++) Gi[(IDX)a.dst[q]] = out[q];
+        if (dup) {
 #pragma unroll
-        for (int q = 0; q < Q; q++) Gi[(IDX)a.dst[q] + 1] = out[q];
+          for (int q = 0; q < Q; q++) Gi[(IDX)a.dst[q] + 1] = out[q];
+        }
       }
     } else if (cat == CAT_EQ) {
 #pragma unroll
@@ -408,8 +498,12 @@ __global__ void __launch_bounds__(STEP_BX, step_min_blocks(EXACT)) k_step(const 
       }
     } else if (dup) {
       // outlet copy of a solid cell in column nx-2: its g is not written this step
+      // (all loads before the stores, which the compiler must assume to alias)
+      S v[Q];
 #pragma unroll
-      for (int q = 0; q < Q; q++) Gi[(IDX)a.dst[q] + 1] = Gi[(IDX)a.dst[q]];
+      for (int q = 0; q < Q; q++) v[q] = Gi[(IDX)a.dst[q]];
+#pragma unroll
+      for (int q = 0; q < Q; q++) Gi[(IDX)a.dst[q] + 1] = v[q];
       if (a.write_fields) {
         a.ux[i + 1] = a.ux[i]; a.uy[i + 1] = a.uy[i]; a.uz[i + 1] = a.uz[i]; a.rho[i + 1] = a.rho[i];
       }

@@ -10,7 +10,7 @@
 // Smagorinsky term depends on |Pi|/rho, which the scale leaves unchanged), so
 // loads and stores carry no scaling multiply. Reciprocals and square roots
 // use the approximate hardware instructions (relative error ~2^-22).
-// patch_raw re-gathers the bounce-back and free-slip directions of one cell
+// patch_raw re-gathers the bounce-back directions of one cell
 // in the same raw units.
 #pragma once
 
@@ -51,16 +51,6 @@ __device__ __forceinline__ float pfma(float a, float b, float c) { return fmaf(a
 __device__ __forceinline__ float prcp(float a) { return rcp_approx(a); }
 __device__ __forceinline__ float psqrt(float a) { return sqrt_approx(a); }
 
-template <int C>
-__device__ __forceinline__ float& lane_of(f2& v) {
-  if constexpr (C == 0) return v.x;
-  else return v.y;
-}
-template <int C>
-__device__ __forceinline__ float& lane_of(float& v) {
-  return v;
-}
-
 // Storage in scaled units: raw(v) is the stored number as a float (the
 // deviation times SC), pack() rounds a pair of raw values to the storage.
 template <class S>
@@ -84,48 +74,30 @@ struct X2<__half> {
   __device__ __forceinline__ static __half to_s(float v) { return __float2half_rn(v); }
 };
 
-// Bounce-back / free-slip re-gather of lane C's cell i, in raw units
-// (js/lbm.js:334-368 for the bounce-back links; k_step's patch_special is
-// the same rule in deviation units). The momentum exchange accumulates in
-// raw units; the caller divides by SC.
-template <class S, int C, class VV>
-__device__ __forceinline__ void patch_raw(const StepArgs<S>& a, long long i, int x, int y, int z,
-                                          bool near_cell, bool shell, VV (&f)[Q], double& Fx,
-                                          double& Fy, double& Fz) {
+// Bounce-back re-gather of a near-wall cell i, in raw units, stationary walls
+// (js/lbm.js:334-368; k_step's patch_bounce is the same rule in deviation
+// units, and loads first and accumulates afterwards for the same reason). The
+// momentum exchange accumulates in raw units; the caller divides by SC.
+template <class S>
+__device__ __forceinline__ void patch_raw(const StepArgs<S>& a, long long i, float (&f)[Q],
+                                          double& Fx, double& Fy, double& Fz) {
   using T = X2<S>;
-  const unsigned long long m = near_cell ? a.nmask[i] : 0ull;
+  const unsigned long long m = a.nmask[i];
   const unsigned sm = (unsigned)m, om = (unsigned)(m >> 32);
-  const float rho_sc = (a.mov && sm ? a.rho[i] : 1.0f) * T::SC;
-#define WT_PATCH_RAW(q)                                                                      \
-  if ((sm >> (q)) & 1u) {                                                                    \
-    const long long j = i - (ex(q) + (long long)ey(q) * a.nx + (long long)ez(q) * a.nxy);    \
-    const float fd = T::raw(a.F[opp(q) * a.n + i]);                                          \
-    float corr = 0.0f;                                                                       \
-    if (a.mov) {                                                                             \
-      const float cu = (float)ex(q) * a.uwx[j] + (float)ey(q) * a.uwy[j] +                   \
-                       (float)ez(q) * a.uwz[j];                                              \
-      if (cu != 0.0f) corr = 6.0f * (float)wq(q) * rho_sc * cu;                              \
-    }                                                                                        \
-    if ((om >> (q)) & 1u) {                                                                  \
-      const float d = 2.0f * fd + corr;                                                      \
-      Fx -= (double)(d * (float)ex(q));                                                      \
-      Fy -= (double)(d * (float)ey(q));                                                      \
-      Fz -= (double)(d * (float)ez(q));                                                      \
-    }                                                                                        \
-    lane_of<C>(f[q]) = fd + corr;                                                            \
-  } else if (shell) {                                                                        \
-    int sy = y - ey(q), sz = z - ez(q), qq = q;                                              \
-    bool refl = false;                                                                       \
-    if (sy == 0 || sy == a.ny - 1) { sy = y; qq = mirror_y(qq); refl = true; }               \
-    if (sz == 0 || sz == a.nz - 1) { sz = z; qq = mirror_z(qq); refl = true; }               \
-    if (refl)                                                                                \
-      lane_of<C>(f[q]) =                                                                     \
-          T::raw(a.F[qq * a.n + (x - ex(q)) + (long long)a.nx * sy + a.nxy * sz]);           \
+#define WT_PATCH_RAW(q) \
+  if ((sm >> (q)) & 1u) f[q] = T::raw(a.F[opp(q) * a.n + i]);
+#define WT_PATCH_FORCE(q)                                                                    \
+  if ((om >> (q)) & 1u) {                                                                    \
+    const float d = 2.0f * f[q];                                                             \
+    Fx -= (double)(d * (float)ex(q));                                                        \
+    Fy -= (double)(d * (float)ey(q));                                                        \
+    Fz -= (double)(d * (float)ez(q));                                                        \
   }
-  WT_PATCH_RAW(1) WT_PATCH_RAW(2) WT_PATCH_RAW(3) WT_PATCH_RAW(4) WT_PATCH_RAW(5)
-  WT_PATCH_RAW(6) WT_PATCH_RAW(7) WT_PATCH_RAW(8) WT_PATCH_RAW(9) WT_PATCH_RAW(10)
-  WT_PATCH_RAW(11) WT_PATCH_RAW(12) WT_PATCH_RAW(13) WT_PATCH_RAW(14) WT_PATCH_RAW(15)
-  WT_PATCH_RAW(16) WT_PATCH_RAW(17) WT_PATCH_RAW(18)
+  WT_EACH_Q(WT_PATCH_RAW)
+  if (om) {
+    WT_EACH_Q(WT_PATCH_FORCE)
+  }
+#undef WT_PATCH_FORCE
 #undef WT_PATCH_RAW
 }
 
