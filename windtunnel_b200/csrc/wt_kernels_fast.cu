@@ -34,6 +34,7 @@ void launch_lean_f16(const StepArgs<__half>& a, dim3 grid, bool, cudaStream_t s)
 // The pair kernel's variant for a lattice, and the grid it runs on.
 template <class S>
 inline int pair_mode(const StepArgs<S>& a) {
+  if (a.sfrac) return PAIR_PBB | (a.nx % 2 ? PAIR_ODD : 0);
   const bool rows = a.nx % (2 * PAIR_BX) == 0 && !a.zfast;
   return (a.nx % 2 ? PAIR_ODD : (rows ? PAIR_ROWS : 0)) | (a.mov ? PAIR_MOV : 0);
 }
@@ -61,6 +62,8 @@ PairKernel<S> pair_kernel(bool sr, int mode) {
       case PAIR_MOV: return k_step_pair<S, false, PAIR_MOV>;
       case PAIR_ODD | PAIR_MOV: return k_step_pair<S, false, PAIR_ODD | PAIR_MOV>;
       case PAIR_ROWS: return k_step_pair<S, false, PAIR_ROWS>;
+      case PAIR_PBB: return k_step_pair<S, false, PAIR_PBB>;
+      case PAIR_PBB | PAIR_ODD: return k_step_pair<S, false, PAIR_PBB | PAIR_ODD>;
       case PAIR_ROWS | PAIR_MOV: return k_step_pair<S, false, PAIR_ROWS | PAIR_MOV>;
       default: return k_step_pair<S, false, 0>;
     }
@@ -94,7 +97,10 @@ void launch_pair_f32(const StepArgs<float>& a, dim3, bool, cudaStream_t s) { lau
 
 // ---- partial bounce-back and adjoint (float32 arithmetic) -------------------------
 
+// The float32 partial-bounce-back step runs the pair kernel (PAIR_PBB), except
+// with moving walls or buffers of 2^31 bytes or more.
 void launch_pbb_f32_fast(const StepArgs<float>& a, dim3 grid, bool wide, cudaStream_t s) {
+  if (!a.mov && 19 * a.n * (long long)sizeof(float) < (1LL << 31)) return launch_pair(a, s);
   if (wide) launch_pdl(k_step_pbb<float, false, long long>, grid, dim3(STEP_BX), s, a);
   else launch_pdl(k_step_pbb<float, false, int>, grid, dim3(STEP_BX), s, a);
 }

@@ -40,6 +40,7 @@
 // srcb / dstb); half storage also needs an even nx and stationary walls.
 #pragma once
 
+#include "wt_pbb.cuh"
 #include "wt_x2.cuh"
 
 namespace wt {
@@ -51,7 +52,8 @@ namespace wt {
 // blocks 8% slower), float32 storage 6 blocks (80 registers, no spills, 24
 // warps; 64-thread blocks 1.5% slower); with an odd nx or moving walls 5, where 6
 // spill (193x85x91: 39.8 against 57.0 us a step; 160x80x80 over a road: 31.0 against
-// 32.9, and 33.6 with 4, in plane order).
+// 32.9, and 33.6 with 4, in plane order); with partial bounce-back 4 (128x64x64, a
+// 32^3 box: 12.9 us a step, 5 blocks 14.4, 6 22.4; the one-cell kernel 18.5).
 constexpr int PAIR_BX = 128;
 
 // Variants of the pair kernel. ODD: an odd nx (float32 storage only): pairs
@@ -61,18 +63,20 @@ constexpr int PAIR_BX = 128;
 // only; the bounce-back correction of js/lbm.js:341-352). ROWS: nx a multiple
 // of 256: each block is an x-segment of one row (grid x, y, z); else the pairs
 // of a plane are numbered along x, then y, across the rows' ends, so that
-// every lane has a pair whatever nx is, for one division per thread.
+// every lane has a pair whatever nx is, for one division per thread. PBB: a
+// partial bounce-back field (wt_pbb.cuh, float32 storage only): the blend of a
+// box cell's outputs with its reversed inputs, and its force.
 // Measured on B200, microseconds a step, one-cell kernels before / pair kernel:
 // 193x85x91 float32 46.3 / 39.8 (ODD against lean); 160x80x80 float32 over a rolling
 // road 40.3 / 28.7 (MOV against direct). Pairs across row ends against one row
 // per block: 64x32x32 float32 8.2 / 6.7 us (three of a block's four warps had
 // nothing to do); on 256x128x128 and 512x192x192 one row per block is 1-2% faster
 // for half storage.
-enum : int { PAIR_ODD = 1, PAIR_MOV = 2, PAIR_ROWS = 4 };
+enum : int { PAIR_ODD = 1, PAIR_MOV = 2, PAIR_ROWS = 4, PAIR_PBB = 8 };
 
 template <class S>
 constexpr int pair_min_blocks(int mode) {
-  return sizeof(S) == 2 ? 7 : (mode & (PAIR_MOV | PAIR_ODD) ? 5 : 6);
+  return sizeof(S) == 2 ? 7 : (mode & PAIR_PBB ? 4 : (mode & (PAIR_MOV | PAIR_ODD) ? 5 : 6));
 }
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
@@ -407,11 +411,14 @@ __device__ __forceinline__ PairCells pair_cells(uint32_t fl, int x0, int nx) {
 }
 
 // Collision of an interior pair whose 19 words are loaded and re-gathered,
-// and the store of its outputs (and, on the last step, its fields).
-template <class S, bool SR, int MODE>
+// and the store of its outputs (and, on the last step, its fields). BLEND: a
+// warp that touches the solid-fraction box, sf the fractions of the two cells
+// (0 for cells that are not computed), F their blend's force before the factor sf.
+template <class S, bool SR, int MODE, bool BLEND>
 __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
                                                    const typename PairIO<S>::W (&w)[Q],
-                                                   long long i0, const PairCells& cells) {
+                                                   long long i0, const PairCells& cells,
+                                                   f2 sf, f2 (&F)[3]) {
   using IO = PairIO<S>;
   using W = typename IO::W;
   using R = typename IO::R;
@@ -425,15 +432,16 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     return *reinterpret_cast<R*>(Gb + a.dstb[q] + sizeof(R) * L);
   };
   // ---- pass 1: moments --------------------------------------------------
-  // ODD and MOV: the moments are summed in trees, the momentum j = r u is
+  // ODD, MOV and PBB: the moments are summed in trees, the momentum j = r u is
   // carried through the update, and the relaxation is added to f instead of
   // scaling f by a rounded 1 - om, so that a step conserves mass and momentum to
   // the rounding of its sums. With the other variants' arithmetic (kept as it
   // is: their results are compared from release to release) the error of u
   // against float64 after 100 steps was 1.3 to 2 times that of the one-cell
-  // kernels these two stand for; so it is 0.3 to 0.6 of theirs (B200, 160x80x80
+  // kernels these stand for; so it is 0.3 to 0.6 of theirs (B200, 160x80x80
   // over a road: uz 1.2e-6 against 1.9e-6; 193x85x91: 7.4e-7 against 1.4e-6).
-  constexpr bool MOM = ODD || MOV;
+  constexpr bool PBB = (MODE & PAIR_PBB) != 0;
+  constexpr bool MOM = ODD || MOV || PBB;
   f2 dr, jx, jy, jz, pxx, pyy, pzz, pxy, pxz, pyz;
   if constexpr (MOM) {
     auto sum = [&](int q) { return padd(IO::to_f2(w[q]), IO::to_f2(w[q + 1])); };
@@ -609,10 +617,14 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     }
   };
   // ---- pass 2: outputs ----------------------------------------------------
+  const f2 s1 = psub(pk(1.0f), sf);   // BLEND only
   {
     const f2 f0 = IO::to_f2(w[0]);
-    if constexpr (MOM)
-      put(0, pfma(om, pfma(pk(12.0f), kae, pmul(pk(-1.0f), f0)), f0));
+    if constexpr (MOM) {
+      f2 g = pfma(om, pfma(pk(12.0f), kae, pmul(pk(-1.0f), f0)), f0);
+      if constexpr (BLEND) g = pfma(sf, f0, pmul(s1, g));
+      put(0, g);
+    }
     else
       put(0, pfma(pfma(pk(-1.0f), om, pk(1.0f)), f0, pmul(pk((float)(1.0 / 3)), omA)));
   }
@@ -625,8 +637,21 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     if constexpr (MOM) {                                            \
       const f2 T = pmul(om, pfma(pk(-0.5f), s, X));                 \
       const f2 U = pfma(pk(-0.5f), d, H);                           \
-      put(qa, padd(fa, pfma(omm, U, T)));                           \
-      put(qa + 1, padd(fb, pfma(pmul(pk(-1.0f), omm), U, T)));      \
+      f2 ga = padd(fa, pfma(omm, U, T));                            \
+      f2 gb = padd(fb, pfma(pmul(pk(-1.0f), omm), U, T));           \
+      if constexpr (BLEND) {                                        \
+        /* c_a (g_a - f_b) + c_b (g_b - f_a), c_b = -c_a */         \
+        const f2 e = padd(psub(ga, gb), d);                         \
+        if constexpr (ex(qa) == 1) F[0] = padd(F[0], e);            \
+        if constexpr (ey(qa) == 1) F[1] = padd(F[1], e);            \
+        if constexpr (ez(qa) == 1) F[2] = padd(F[2], e);            \
+        if constexpr (ey(qa) == -1) F[1] = psub(F[1], e);           \
+        if constexpr (ez(qa) == -1) F[2] = psub(F[2], e);           \
+        ga = pfma(sf, fb, pmul(s1, ga));                            \
+        gb = pfma(sf, fa, pmul(s1, gb));                            \
+      }                                                             \
+      put(qa, ga);                                                  \
+      put(qa + 1, gb);                                              \
     } else {                                                        \
       const f2 Y = pmul(K3, c);                                     \
       const f2 P = pfma(al, s, X), M = pfma(be, d, Y);              \
@@ -668,7 +693,7 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
   using W = typename IO::W;
   constexpr float SC = IO::SC;
   constexpr bool ODD = (MODE & PAIR_ODD) != 0, MOV = (MODE & PAIR_MOV) != 0;
-  constexpr bool ROWS = (MODE & PAIR_ROWS) != 0;
+  constexpr bool ROWS = (MODE & PAIR_ROWS) != 0, PBB = (MODE & PAIR_PBB) != 0;
   int x0, y, z;
   if constexpr (ROWS) {
     x0 = 2 * (int)(blockIdx.x * PAIR_BX + threadIdx.x);
@@ -684,15 +709,15 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
   const bool edge = z == 0 || z == a.nz - 1 || y >= a.ny - 1 || y == 0;
   pdl_enter();   // programmatic dependent launch (launch_pdl)
   if (edge) {
-    // rows that pull nothing; they hold no near-wall cell, so no force partial
+    // rows that pull nothing and hold no near-wall cell
     if (ROWS || y < a.ny) {
       if constexpr (ODD) pair_edge_row_odd<S>(a, i0, x0, y, z);
       else pair_edge_row<S>(a, i0, x0, y, z);
     }
-    if constexpr (ROWS) return;
+    if constexpr (ROWS && !PBB) return;
   }
-  const bool active = ROWS || !edge;
-  if (!ROWS && __all_sync(0xffffffffu, edge)) return;
+  const bool active = (ROWS && !PBB) || !edge;
+  if (!(ROWS || PBB) && __all_sync(0xffffffffu, edge)) return;
   // interior row: pull every direction of both cells. The sources of the
   // pair (x0 - ex, x0 + 1 - ex) of row (y - ey, z - ez) lie inside the
   // buffer for every cell of an interior row.
@@ -726,6 +751,13 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
   WT_EACH_Q(WT_PAIR_JOIN)
 #undef WT_PAIR_JOIN
   const PairCells c = pair_cells<MODE>(fl, x0, a.nx);
+  const long long seg = ROWS ? seg_of(x0, y, z, a.nx, a.ny)
+                             : (long long)plane_of(a) * segs_per_plane(a.nx, a.ny) +
+                                   (block_of(a) * (PAIR_BX / 16) + (threadIdx.x >> 4));
+  // a segment that touches the solid-fraction box writes its partial every
+  // step: the pair takes part in it if any of its cells lies in the box
+  const bool in_box = PBB && x0 < a.sb[3] && x0 + (ODD && x0 == a.nx - 3 ? 2 : 1) >= a.sb[0] &&
+                      y >= a.sb[1] && y < a.sb[4] && z >= a.sb[2] && z < a.sb[5];
   {
     // the momentum exchange of the re-gathered body links, summed per
     // 32-cell segment here, so that its doubles are not live across the
@@ -734,14 +766,43 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
     if (active && c.near0) pair_patch<S, MOV>(a, i0, 0, w, Fx, Fy, Fz);
     if (active && c.near1) pair_patch<S, MOV>(a, i0 + 1, 1, w, Fx, Fy, Fz);
     constexpr double inv_sc = 1.0 / (double)SC;   // a power of two: exact
-    const long long seg =
-        ROWS ? seg_of(x0, y, z, a.nx, a.ny)
-             : (long long)plane_of(a) * segs_per_plane(a.nx, a.ny) +
-                   (block_of(a) * (PAIR_BX / 16) + (threadIdx.x >> 4));
-    pair_force_partial(Fx * inv_sc, Fy * inv_sc, Fz * inv_sc, active && (c.near0 || c.near1), a,
-                       seg);
+    pair_force_partial(Fx * inv_sc, Fy * inv_sc, Fz * inv_sc,
+                       (active && (c.near0 || c.near1)) || in_box, a, seg);
   }
-  if (active) pair_collide_store<S, SR, MODE>(a, w, i0, c);
+  f2 sf = pk(0.0f), F[3] = {pk(0.0f), pk(0.0f), pk(0.0f)};
+  const bool blend = PBB && __any_sync(0xffffffffu, in_box);
+  if (PBB && blend && in_box) {
+    if (c.fluid0) sf.x = (float)sfrac_at(a, x0, y, z);
+    if (c.fluid1) sf.y = (float)sfrac_at(a, x0 + 1, y, z);
+  }
+  if (blend) {
+    if (active) pair_collide_store<S, SR, MODE, PBB>(a, w, i0, c, sf, F);
+  } else {
+    if (active) pair_collide_store<S, SR, MODE, false>(a, w, i0, c, sf, F);
+  }
+  if (PBB && blend) {
+    // the blend's force joins the partial that this half-warp's first lane stored
+    const f2 fx = pmul(sf, F[0]), fy = pmul(sf, F[1]), fz = pmul(sf, F[2]);
+    constexpr double inv_sc = 1.0 / (double)SC;
+    double px = ((double)fx.x + (double)fx.y) * inv_sc, py = ((double)fy.x + (double)fy.y) * inv_sc,
+           pz = ((double)fz.x + (double)fz.y) * inv_sc;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      px += __shfl_down_sync(0xffffffffu, px, o, 16);
+      py += __shfl_down_sync(0xffffffffu, py, o, 16);
+      pz += __shfl_down_sync(0xffffffffu, pz, o, 16);
+    }
+    const unsigned boxes = __ballot_sync(0xffffffffu, in_box);
+    const unsigned lane = threadIdx.x & 31u;
+    if ((lane & 15u) == 0u && ((boxes >> lane) & 0xffffu) != 0u) {
+      const int slot = a.wslot[seg];
+      if (slot >= 0) {
+        a.part[3 * (size_t)slot] += px;
+        a.part[3 * (size_t)slot + 1] += py;
+        a.part[3 * (size_t)slot + 2] += pz;
+      }
+    }
+  }
 }
 
 }  // namespace wt
