@@ -68,12 +68,13 @@ long long range_cells(const int rg[6]) {
 
 void free_all(wt_lattice* h) {
   void* dev[] = {h->buf[0], h->buf[1], h->flags, h->nmask, h->ux, h->uy, h->uz, h->rho, h->uwx, h->uwy,
-                 h->uwz, h->part, h->wslot, h->forces_dev, h->err_dev, h->col, h->plan, h->low,
-                 h->counters};
+                 h->uwz, h->part, h->wslot, h->segmark, h->slot_scan, h->sfrac_buf, h->err_dev,
+                 h->vstats, h->vox_in};
   for (void* p : dev)
     if (p) cudaFree(p);
   if (h->forces_host) cudaFreeHost(h->forces_host);
   if (h->err_host) cudaFreeHost(h->err_host);
+  if (h->stage) cudaFreeHost(h->stage);
   if (h->stream) cudaStreamDestroy(h->stream);
   if (h->aux) cudaStreamDestroy(h->aux);
   if (h->adj_pool) cudaFree(h->adj_pool);
@@ -98,18 +99,35 @@ int check_params(const wt_params* p) {
 int grow_forces(wt_lattice* h, int nsteps) {
   if (nsteps <= h->forces_cap) return WT_OK;
   int cap = std::max(nsteps, 2 * h->forces_cap);
-  if (h->forces_dev) cudaFree(h->forces_dev);
   if (h->forces_host) cudaFreeHost(h->forces_host);
-  h->forces_dev = nullptr;
   h->forces_host = nullptr;
   h->forces_cap = 0;
-  if (cudaMalloc(&h->forces_dev, sizeof(double) * 3 * (size_t)cap) != cudaSuccess)
-    return fail(h, WT_ERR_OOM, "cannot allocate the device force series");
   if (cudaMallocHost(&h->forces_host, sizeof(double) * 3 * (size_t)cap) != cudaSuccess)
     return fail(h, WT_ERR_OOM, "cannot allocate the pinned force series");
   h->forces_cap = cap;
   return WT_OK;
 }
+
+}  // namespace
+
+void* wt::stage(wt_lattice* h, size_t bytes) {
+  if (bytes > kStageMax) return nullptr;
+  if (bytes > h->stage_bytes) {
+    const size_t cap = std::max<size_t>(2 * bytes, 1 << 16);
+    if (h->stage) cudaFreeHost(h->stage);
+    h->stage = nullptr;
+    h->stage_bytes = 0;
+    if (cudaMallocHost(&h->stage, cap) != cudaSuccess) {
+      cudaGetLastError();
+      h->stage = nullptr;
+      return nullptr;
+    }
+    h->stage_bytes = cap;
+  }
+  return h->stage;
+}
+
+namespace {
 
 template <class S>
 S to_store(double v);
@@ -180,11 +198,12 @@ template <class S>
 using StepLaunch = void (*)(const wt::StepArgs<S>&, dim3, bool, cudaStream_t);
 
 // nsteps steps of one kernel: the force partials of up to `chunk` steps go to
-// `part` (one block of slots per step) and are reduced into forces_dev once
-// per chunk; error bits go to `err`.
+// `part` (one block of slots per step) and are reduced into forces_dev (device
+// or pinned host memory) once per chunk; error bits go to `err`, and with
+// err_out from there to err_out at the end of the call, `err` being zeroed.
 template <class S>
 void run_steps(wt_lattice* h, int nsteps, StepLaunch<S> launch, double* part, double* forces_dev,
-               unsigned* err, int chunk_max) {
+               unsigned* err, unsigned* err_out, int chunk_max) {
   wt::StepArgs<S> a = make_args<S>(h);
   a.err = err;
   const dim3 grid = wt::step_grid(a);
@@ -202,8 +221,8 @@ void run_steps(wt_lattice* h, int nsteps, StepLaunch<S> launch, double* part, do
       h->launches++;
       h->parity ^= 1;
     }
-    wt::launch_force_reduce(part, (unsigned)h->nslots, chunk, forces_dev + 3 * (size_t)done,
-                            h->stream);
+    wt::launch_force_reduce(part, (unsigned)h->nslots, chunk, forces_dev + 3 * (size_t)done, err,
+                            done + chunk == nsteps ? err_out : nullptr, h->stream);
     h->launches++;
     done += chunk;
   }
@@ -250,38 +269,20 @@ bool pair_auto(const wt_lattice* h) {
 
 int select_path(wt_lattice* h, Path* out);
 void dispatch_steps(wt_lattice* h, int nsteps, Path path, double* part, double* forces_dev,
-                    unsigned* err, int chunk);
+                    unsigned* err, unsigned* err_out, int chunk);
 int check_err_word(wt_lattice* h, unsigned word);
 
-// Assign a force-partial slot to every 32-cell segment that holds a
-// near-wall cell (js/lbm.js:334-359 only accumulates there) and size the
-// partial buffer.
+// Assign a force-partial slot to every 32-cell segment that holds a near-wall
+// cell (js/lbm.js:334-359 only accumulates there) or touches the solid-fraction
+// box, and size the partial buffer. Ends with a synchronisation of the stream.
 int rebuild_slots(wt_lattice* h) {
-  uint8_t* mark = nullptr;
-  if (cudaMalloc(&mark, (size_t)h->nsegs) != cudaSuccess)
-    return fail(h, WT_ERR_OOM, "cannot allocate the warp marks");
-  std::vector<uint8_t> hm((size_t)h->nsegs);
-  cudaError_t e = cudaMemsetAsync(mark, 0, (size_t)h->nsegs, h->stream);
-  if (e == cudaSuccess) {
-    wt::launch_mark_segments(h->flags, h->nx, h->ny, h->nz, mark, h->stream);
-    h->launches++;
-    e = cudaMemcpyAsync(hm.data(), mark, hm.size(), cudaMemcpyDeviceToHost, h->stream);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  cudaFree(mark);
-  if (e != cudaSuccess) return cuda_fail(h, e, "rebuild_slots");
-  if (h->sfrac) {
-    // every segment that touches the partial bounce-back box carries a force partial
-    const int* b = h->sbox;
-    for (int z = b[2]; z < b[5]; z++)
-      for (int y = b[1]; y < b[4]; y++) {
-        const long long s1 = wt::seg_of(b[3] - 1, y, z, h->nx, h->ny);
-        for (long long s = wt::seg_of(b[0], y, z, h->nx, h->ny); s <= s1; s++) hm[(size_t)s] = 1;
-      }
-  }
-  std::vector<int> slot(hm.size());
+  wt::launch_slots(h);
   int n = 0;
-  for (size_t w = 0; w < hm.size(); w++) slot[w] = hm[w] ? n++ : -1;
+  cudaError_t e = cudaMemcpyAsync(&n, h->slot_scan + wt::slot_scan_ints(h) - 1, sizeof(int),
+                                  cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(h, e, "rebuild_slots");
   if (n > h->part_cap || !h->part) {
     if (h->part) cudaFree(h->part);
     h->part = nullptr;
@@ -291,12 +292,34 @@ int rebuild_slots(wt_lattice* h) {
       return fail(h, WT_ERR_OOM, "cannot allocate the force partials");
     h->part_cap = cap;
   }
-  e = cudaMemcpyAsync(h->wslot, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice,
-                      h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e != cudaSuccess) return cuda_fail(h, e, "rebuild_slots upload");
   h->nslots = n;
   return WT_OK;
+}
+
+// Device room for voxelize's inputs: kept in the handle up to kVoxKeep bytes
+// (a body dragged through the lattice then allocates nothing), else given back
+// by vox_in_done.
+constexpr size_t kVoxKeep = 64u << 20;
+
+void* vox_in(wt_lattice* h, size_t bytes) {
+  if (bytes > h->vox_in_bytes) {
+    if (h->vox_in) cudaFree(h->vox_in);
+    h->vox_in = nullptr;
+    h->vox_in_bytes = 0;
+    if (cudaMalloc(&h->vox_in, bytes) != cudaSuccess) {
+      h->vox_in = nullptr;
+      return nullptr;
+    }
+    h->vox_in_bytes = bytes;
+  }
+  return h->vox_in;
+}
+
+void vox_in_done(wt_lattice* h) {
+  if (h->vox_in_bytes <= kVoxKeep) return;
+  cudaFree(h->vox_in);
+  h->vox_in = nullptr;
+  h->vox_in_bytes = 0;
 }
 
 }  // namespace
@@ -388,10 +411,14 @@ int wt_create(int nx, int ny, int nz, int storage, wt_lattice** out) {
   ok = ok && cudaMalloc((void**)&h->wslot, sizeof(int) * (size_t)h->nsegs) == cudaSuccess;
   ok = ok && cudaMalloc((void**)&h->err_dev, sizeof(unsigned)) == cudaSuccess;
   ok = ok && cudaMallocHost((void**)&h->err_host, sizeof(unsigned)) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->col, (size_t)ny * nz) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->plan, (size_t)nx * nz) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->low, sizeof(int) * (size_t)nx * nz) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->counters, sizeof(int) * 2) == cudaSuccess;
+  ok = ok && cudaMalloc((void**)&h->segmark, (size_t)h->nsegs) == cudaSuccess;
+  ok = ok && cudaMalloc((void**)&h->slot_scan, sizeof(int) * wt::slot_scan_ints(h)) == cudaSuccess;
+  h->vstats_bytes = 8 + 5 * (size_t)nx * nz + (size_t)ny * nz;
+  ok = ok && cudaMalloc((void**)&h->vstats, h->vstats_bytes) == cudaSuccess;
+  h->counters = (int*)h->vstats;
+  h->low = h->counters + 2;
+  h->col = (uint8_t*)(h->low + (size_t)nx * nz);
+  h->plan = h->col + (size_t)ny * nz;
   ok = ok && grow_forces(h, 64) == WT_OK;
   if (!ok) {
     cudaGetLastError();
@@ -402,7 +429,8 @@ int wt_create(int nx, int ny, int nz, int storage, wt_lattice** out) {
     return WT_ERR_OOM;
   }
   cudaMemsetAsync(h->flags, 0, (size_t)n, h->stream);
-  cudaMemsetAsync(h->nmask, 0, sizeof(unsigned long long) * (size_t)n, h->stream);
+  cudaMemsetAsync(h->segmark, 0, (size_t)h->nsegs, h->stream);
+  cudaMemsetAsync(h->err_dev, 0, sizeof(unsigned), h->stream);
   for (float* p : {h->uwx, h->uwy, h->uwz}) cudaMemsetAsync(p, 0, sizeof(float) * n, h->stream);
   wt::launch_init(h, 0, 0, 0);
   cudaError_t e = cudaStreamSynchronize(h->stream);
@@ -483,53 +511,58 @@ int wt_voxel_range(const wt_lattice* h, const double box[6], int range[6]) {
 
 namespace {
 
-// Shared tail of both voxelize forms: statistics and near flags.
-int voxelize_finish(wt_lattice* h, int ground, double road_vel) {
-  std::vector<uint8_t> col((size_t)h->ny * h->nz), plan((size_t)h->nx * h->nz);
-  std::vector<int> low((size_t)h->nx * h->nz);
-  int counters[2] = {0, 0};
-  WT_CUDA(h, cudaMemcpyAsync(col.data(), h->col, col.size(), cudaMemcpyDeviceToHost, h->stream));
-  WT_CUDA(h, cudaMemcpyAsync(plan.data(), h->plan, plan.size(), cudaMemcpyDeviceToHost, h->stream));
-  WT_CUDA(h, cudaMemcpyAsync(low.data(), h->low, sizeof(int) * low.size(), cudaMemcpyDeviceToHost,
-                             h->stream));
-  WT_CUDA(h, cudaMemcpyAsync(counters, h->counters, sizeof(counters), cudaMemcpyDeviceToHost,
-                             h->stream));
-  wt::launch_near(h);
-  WT_CUDA(h, cudaStreamSynchronize(h->stream));
-  WT_CUDA(h, cudaGetLastError());
-  // js/lbm.js:247-264
+// The body's reference statistics (js/lbm.js:247-264) from the projections.
+void voxelize_stats(wt_lattice* h, const unsigned char* v, int ground, double road_vel) {
+  const size_t nc = (size_t)h->ny * h->nz, np = (size_t)h->nx * h->nz;
+  int counters[2];
+  memcpy(counters, v, sizeof(counters));
+  const int* low = (const int*)(v + sizeof(counters));
+  const uint8_t* col = (const uint8_t*)(low + np);
+  const uint8_t* plan = col + nc;
   long long a = 0, pa = 0;
-  for (uint8_t v : col) a += v;
-  for (uint8_t v : plan) pa += v;
+  for (size_t k = 0; k < nc; k++) a += col[k];
+  for (size_t k = 0; k < np; k++) pa += plan[k];
   std::vector<int> gaps;
-  for (size_t k = 0; k < plan.size(); k++) {
+  for (size_t k = 0; k < np; k++) {
     if (plan[k] && low[k] < 32767) {
       const int g = low[k] - 1;
       if (g > 0) gaps.push_back(g);
     }
   }
-  std::sort(gaps.begin(), gaps.end());
+  h->stats.ride_height = 0;
+  if (!gaps.empty()) {
+    auto mid = gaps.begin() + (gaps.size() >> 1);
+    std::nth_element(gaps.begin(), mid, gaps.end());
+    h->stats.ride_height = *mid;
+  }
   h->stats.frontal_area = (int)std::max<long long>(1, a);
   h->stats.planform_area = (int)std::max<long long>(1, pa);
   h->stats.solid_cells = counters[0];
-  h->stats.ride_height = gaps.empty() ? 0 : gaps[gaps.size() >> 1];
   h->stats.ground = ground ? 1 : 0;
   h->p.moving_walls = (road_vel != 0 || counters[1]) ? 1 : 0;
   h->stats.moving_walls = h->p.moving_walls;
-  return rebuild_slots(h);
+}
+
+// Shared tail of both voxelize forms: near flags, slots, statistics. The whole
+// of voxelize is one sequence on the stream up to here; rebuild_slots waits.
+int voxelize_finish(wt_lattice* h, int ground, double road_vel) {
+  wt::launch_near(h);
+  const int c = rebuild_slots(h);
+  if (c != WT_OK) return c;
+  std::vector<unsigned char> v(h->vstats_bytes);
+  WT_CUDA(h, cudaMemcpyAsync(v.data(), h->vstats, v.size(), cudaMemcpyDeviceToHost, h->stream));
+  WT_CUDA(h, cudaStreamSynchronize(h->stream));
+  voxelize_stats(h, v.data(), ground, road_vel);
+  return WT_OK;
 }
 
 int voxelize_start(wt_lattice* h, int ground, double road_vel) {
   wt::launch_clear_obj(h);
   wt::launch_floor(h, ground, road_vel);
-  std::vector<int> low((size_t)h->nx * h->nz, 32767);
-  WT_CUDA(h, cudaMemsetAsync(h->col, 0, (size_t)h->ny * h->nz, h->stream));
-  WT_CUDA(h, cudaMemsetAsync(h->plan, 0, (size_t)h->nx * h->nz, h->stream));
-  WT_CUDA(h, cudaMemcpyAsync(h->low, low.data(), sizeof(int) * low.size(), cudaMemcpyHostToDevice,
-                             h->stream));
-  WT_CUDA(h, cudaMemsetAsync(h->counters, 0, sizeof(int) * 2, h->stream));
-  // the host vector must outlive the async copy
-  WT_CUDA(h, cudaStreamSynchronize(h->stream));
+  WT_CUDA(h, cudaMemsetAsync(h->vstats, 0, h->vstats_bytes, h->stream));
+  // no body cell in the column: any value above 32767 (a lowest cell of 32767 or
+  // more counts as none, js/lbm.js:257)
+  WT_CUDA(h, cudaMemsetAsync(h->low, 0x7f, sizeof(int) * (size_t)h->nx * h->nz, h->stream));
   return WT_OK;
 }
 
@@ -552,28 +585,29 @@ int wt_voxelize_mask(wt_lattice* h, const double box[6], const uint8_t* inside, 
   int c = voxelize_start(h, ground, road_vel);
   if (c != WT_OK) return c;
   if (cells > 0) {
-    uint8_t* mask_dev = nullptr;
-    uint8_t* ws_dev = nullptr;
-    double* wv_dev = nullptr;
-    cudaError_t e = cudaMalloc(&mask_dev, (size_t)cells);
-    if (e == cudaSuccess && wall_set) e = cudaMalloc(&ws_dev, (size_t)cells);
-    if (e == cudaSuccess && wall_set) e = cudaMalloc(&wv_dev, sizeof(double) * 3 * (size_t)cells);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(mask_dev, inside, (size_t)cells, cudaMemcpyHostToDevice, h->stream);
+    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    const size_t sz = up((size_t)cells);
+    uint8_t* mask_dev =
+        (uint8_t*)vox_in(h, sz + (wall_set ? sz + sizeof(double) * 3 * (size_t)cells : 0));
+    if (!mask_dev) {
+      cudaGetLastError();
+      return fail(h, WT_ERR_CUDA, "voxelize: out of memory");
+    }
+    uint8_t* ws_dev = wall_set ? mask_dev + sz : nullptr;
+    double* wv_dev = wall_set ? (double*)(mask_dev + 2 * sz) : nullptr;
+    cudaError_t e = cudaMemcpyAsync(mask_dev, inside, (size_t)cells, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess && wall_set)
       e = cudaMemcpyAsync(ws_dev, wall_set, (size_t)cells, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess && wall_set)
       e = cudaMemcpyAsync(wv_dev, wall_vel, sizeof(double) * 3 * (size_t)cells,
                           cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) wt::launch_box_mask(h, rg, mask_dev, ws_dev, wv_dev);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (mask_dev) cudaFree(mask_dev);
-    if (ws_dev) cudaFree(ws_dev);
-    if (wv_dev) cudaFree(wv_dev);
     if (e != cudaSuccess) return cuda_fail(h, e, "voxelize");
   }
-  return voxelize_finish(h, ground, road_vel);
+  c = voxelize_finish(h, ground, road_vel);
+  vox_in_done(h);
+  return c;
 }
 
 int wt_voxelize_grid(wt_lattice* h, const uint8_t* grid, int gnx, int gny, int gnz,
@@ -590,18 +624,20 @@ int wt_voxelize_grid(wt_lattice* h, const uint8_t* grid, int gnx, int gny, int g
   if (c != WT_OK) return c;
   if (cells > 0) {
     const size_t gbytes = (size_t)gnx * gny * gnz;
-    uint8_t* grid_dev = nullptr;
-    cudaError_t e = cudaMalloc(&grid_dev, gbytes);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(grid_dev, grid, gbytes, cudaMemcpyHostToDevice, h->stream);
+    uint8_t* grid_dev = (uint8_t*)vox_in(h, gbytes);
+    if (!grid_dev) {
+      cudaGetLastError();
+      return fail(h, WT_ERR_CUDA, "voxelize_grid: out of memory");
+    }
+    cudaError_t e = cudaMemcpyAsync(grid_dev, grid, gbytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess)
       wt::launch_box_grid(h, rg, grid_dev, gnx, gny, gnz, gmin, ginv, M, P, scale);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (grid_dev) cudaFree(grid_dev);
     if (e != cudaSuccess) return cuda_fail(h, e, "voxelize_grid");
   }
-  return voxelize_finish(h, ground, road_vel);
+  c = voxelize_finish(h, ground, road_vel);
+  vox_in_done(h);
+  return c;
 }
 
 int wt_get_body_stats(const wt_lattice* h, wt_body_stats* out) {
@@ -617,16 +653,14 @@ int wt_step(wt_lattice* h, int nsteps, double* forces) {
   if (nsteps == 0) return WT_OK;
   int c = grow_forces(h, nsteps);
   if (c != WT_OK) return c;
-  WT_CUDA(h, cudaMemsetAsync(h->err_dev, 0, sizeof(unsigned), h->stream));
   Path path = Path::Direct;
   c = select_path(h, &path);
   if (c != WT_OK) return c;
-  dispatch_steps(h, nsteps, path, h->part, h->forces_dev, h->err_dev, kChunk);
+  // The reduction writes the forces and the error word to pinned memory: a
+  // call is its steps, one reduction per chunk and one wait (with a memset and
+  // two copies around them a single step of a small lattice took 34 us).
+  dispatch_steps(h, nsteps, path, h->part, h->forces_host, h->err_dev, h->err_host, kChunk);
   WT_CUDA(h, cudaGetLastError());
-  WT_CUDA(h, cudaMemcpyAsync(h->forces_host, h->forces_dev, sizeof(double) * 3 * (size_t)nsteps,
-                             cudaMemcpyDeviceToHost, h->stream));
-  WT_CUDA(h, cudaMemcpyAsync(h->err_host, h->err_dev, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                             h->stream));
   WT_CUDA(h, cudaStreamSynchronize(h->stream));
   h->steps += nsteps;
   const double* last = h->forces_host + 3 * (size_t)(nsteps - 1);
@@ -687,7 +721,7 @@ StepLaunch<S> pick(Path path, StepLaunch<S> direct, StepLaunch<S> lean, StepLaun
 
 // Run nsteps steps of the chosen kernel; per-step forces land in forces_dev.
 void dispatch_steps(wt_lattice* h, int nsteps, Path path, double* part, double* forces_dev,
-                    unsigned* err, int chunk) {
+                    unsigned* err, unsigned* err_out, int chunk) {
   const bool exact = h->p.math == WT_MATH_EXACT || h->storage == WT_STORE_F64;
   switch (h->storage) {
     case WT_STORE_F32:
@@ -695,24 +729,24 @@ void dispatch_steps(wt_lattice* h, int nsteps, Path path, double* part, double* 
         run_steps<float>(h, nsteps,
                          pick<float>(path, wt::launch_step_f32_exact, wt::launch_step_f32_exact,
                                      wt::launch_pbb_f32_exact),
-                         part, forces_dev, err, chunk);
+                         part, forces_dev, err, err_out, chunk);
       else
         run_steps<float>(h, nsteps,
                          pick<float>(path, wt::launch_step_f32_fast, wt::launch_lean_f32,
                                      wt::launch_pbb_f32_fast, wt::launch_pair_f32),
-                         part, forces_dev, err, chunk);
+                         part, forces_dev, err, err_out, chunk);
       break;
     case WT_STORE_F16DEV:
       run_steps<__half>(h, nsteps,
                         pick<__half>(path, wt::launch_step_f16_fast, wt::launch_lean_f16,
                                      wt::launch_pbb_f16_fast, wt::launch_pair_f16),
-                        part, forces_dev, err, chunk);
+                        part, forces_dev, err, err_out, chunk);
       break;
     default:
       run_steps<double>(h, nsteps,
                         pick<double>(path, wt::launch_step_f64_exact, wt::launch_step_f64_exact,
                                      wt::launch_pbb_f64_exact),
-                        part, forces_dev, err, chunk);
+                        part, forces_dev, err, err_out, chunk);
       break;
   }
 }
@@ -758,19 +792,19 @@ int wt_get_fields(wt_lattice* h, float* ux, float* uy, float* uz, float* rho) {
 
 int wt_get_solid(wt_lattice* h, uint8_t* out) {
   if (!h || !out) return WT_ERR_ARG;
-  std::vector<uint8_t> fl((size_t)h->n);
-  WT_CUDA(h, cudaMemcpyAsync(fl.data(), h->flags, fl.size(), cudaMemcpyDeviceToHost, h->stream));
+  WT_CUDA(h, cudaMemcpyAsync(out, h->flags, (size_t)h->n, cudaMemcpyDeviceToHost, h->stream));
   WT_CUDA(h, cudaStreamSynchronize(h->stream));
-  for (size_t i = 0; i < fl.size(); i++) out[i] = fl[i] & wt::FLAG_SOLID_MASK;
+  const size_t n = (size_t)h->n;   // not through h, which out might alias
+  for (size_t i = 0; i < n; i++) out[i] &= wt::FLAG_SOLID_MASK;
   return WT_OK;
 }
 
 int wt_get_near(wt_lattice* h, uint8_t* out) {
   if (!h || !out) return WT_ERR_ARG;
-  std::vector<uint8_t> fl((size_t)h->n);
-  WT_CUDA(h, cudaMemcpyAsync(fl.data(), h->flags, fl.size(), cudaMemcpyDeviceToHost, h->stream));
+  WT_CUDA(h, cudaMemcpyAsync(out, h->flags, (size_t)h->n, cudaMemcpyDeviceToHost, h->stream));
   WT_CUDA(h, cudaStreamSynchronize(h->stream));
-  for (size_t i = 0; i < fl.size(); i++) out[i] = (fl[i] & wt::FLAG_NEAR) ? 1 : 0;
+  const size_t n = (size_t)h->n;
+  for (size_t i = 0; i < n; i++) out[i] = (out[i] & wt::FLAG_NEAR) ? 1 : 0;
   return WT_OK;
 }
 
@@ -914,6 +948,16 @@ int wt_sample(wt_lattice* h, const double* xyz, int npts, double* out) {
   if (!h) return WT_ERR_ARG;
   if (npts < 0 || (npts > 0 && (!xyz || !out))) return fail(h, WT_ERR_ARG, "bad points");
   if (npts == 0) return WT_OK;
+  const size_t bytes = sizeof(double) * 3 * (size_t)npts;
+  if (double* p = (double*)wt::stage(h, 2 * bytes)) {   // in place, in pinned memory
+    memcpy(p, xyz, bytes);
+    wt::launch_sample(h, p, npts, p + 3 * (size_t)npts);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return cuda_fail(h, e, "sample");
+    memcpy(out, p + 3 * (size_t)npts, bytes);
+    return WT_OK;
+  }
   double* d = nullptr;
   if (cudaMalloc(&d, sizeof(double) * 6 * (size_t)npts) != cudaSuccess)
     return fail(h, WT_ERR_OOM, "sample buffer");
@@ -964,10 +1008,7 @@ int wt_get_launch_count(const wt_lattice* h, int64_t* count) {
 
 extern "C" int wt_set_solid_fraction(wt_lattice* h, const int box[6], const double* s) {
   if (!h) return WT_ERR_ARG;
-  if (h->sfrac) {
-    cudaFree(h->sfrac);
-    h->sfrac = nullptr;
-  }
+  h->sfrac = nullptr;
   for (int k = 0; k < 6; k++) h->sbox[k] = 0;
   if (!box) return rebuild_slots(h);
   const int x0 = box[0], y0 = box[1], z0 = box[2], x1 = box[3], y1 = box[4], z1 = box[5];
@@ -976,14 +1017,22 @@ extern "C" int wt_set_solid_fraction(wt_lattice* h, const int box[6], const doub
     return fail(h, WT_ERR_ARG, "solid-fraction box must be non-empty and inside the lattice, "
                                "with values");
   const size_t m = (size_t)(x1 - x0) * (y1 - y0) * (z1 - z0);
-  for (size_t k = 0; k < m; k++)
-    if (!std::isfinite(s[k]) || s[k] < 0.0 || s[k] > 1.0)
-      return fail(h, WT_ERR_ARG, "solid fractions must lie in [0, 1]");
-  if (cudaMalloc((void**)&h->sfrac, sizeof(double) * m) != cudaSuccess) {
-    h->sfrac = nullptr;
-    return fail(h, WT_ERR_OOM, "cannot allocate the solid-fraction field");
+  size_t bad = 0;
+  for (size_t k = 0; k < m; k++) bad += !(s[k] >= 0.0 && s[k] <= 1.0);   // NaN and infinities too
+  if (bad) return fail(h, WT_ERR_ARG, "solid fractions must lie in [0, 1]");
+  if (m > h->sfrac_cap) {
+    if (h->sfrac_buf) cudaFree(h->sfrac_buf);
+    h->sfrac_buf = nullptr;
+    h->sfrac_cap = 0;
+    if (cudaMalloc((void**)&h->sfrac_buf, sizeof(double) * m) != cudaSuccess) {
+      h->sfrac_buf = nullptr;
+      cudaGetLastError();
+      return fail(h, WT_ERR_OOM, "cannot allocate the solid-fraction field");
+    }
+    h->sfrac_cap = m;
   }
-  WT_CUDA(h, cudaMemcpy(h->sfrac, s, sizeof(double) * m, cudaMemcpyHostToDevice));
+  WT_CUDA(h, cudaMemcpyAsync(h->sfrac_buf, s, sizeof(double) * m, cudaMemcpyHostToDevice, h->stream));
+  h->sfrac = h->sfrac_buf;
   for (int k = 0; k < 6; k++) h->sbox[k] = box[k];
   return rebuild_slots(h);
 }
@@ -1108,7 +1157,7 @@ int adjoint_run(wt_lattice* h, const wt_adj_cfg& cfg, int C, double* dJds, wt_ad
   for (int k = 0; k + 1 < ncp; k++) {
     WT_CUDA(h, cudaMemcpyAsync(cps + (size_t)k * pel, h->buf[h->parity], pop,
                                cudaMemcpyDeviceToDevice, h->stream));
-    dispatch_steps(h, C, Path::Pbb, h->part, fdev + 3 * (size_t)k * C, h->err_dev, kChunk);
+    dispatch_steps(h, C, Path::Pbb, h->part, fdev + 3 * (size_t)k * C, h->err_dev, nullptr, kChunk);
   }
   const int tl = (ncp - 1) * C, nl = N - tl;   // the last interval
   S* last = seg[(ncp - 1) & 1];
@@ -1128,7 +1177,7 @@ int adjoint_run(wt_lattice* h, const wt_adj_cfg& cfg, int C, double* dJds, wt_ad
         h->launches++;
       }
       wt::launch_force_reduce(h->part, (unsigned)h->nslots, chunk,
-                              fdev + 3 * ((size_t)tl + done), h->stream);
+                              fdev + 3 * ((size_t)tl + done), h->err_dev, nullptr, h->stream);
       h->launches++;
       done += chunk;
     }
@@ -1187,6 +1236,7 @@ int adjoint_run(wt_lattice* h, const wt_adj_cfg& cfg, int C, double* dJds, wt_ad
   WT_CUDA(h, cudaMemcpyAsync(dJds, ds, sizeof(double) * nbox, cudaMemcpyDeviceToHost, h->stream));
   WT_CUDA(h, cudaMemcpyAsync(h->err_host, h->err_dev, sizeof(unsigned), cudaMemcpyDeviceToHost,
                              h->stream));
+  WT_CUDA(h, cudaMemsetAsync(h->err_dev, 0, sizeof(unsigned), h->stream));
   WT_CUDA(h, cudaStreamSynchronize(h->stream));
   float fwd_ms = 0, bwd_ms = 0;
   cudaEventElapsedTime(&fwd_ms, e0, e1);
@@ -1323,7 +1373,7 @@ extern "C" int wt_step_noalloc(wt_lattice* h, int nsteps, double* forces) {
   // Only the error word must start at zero: every used partial slot and
   // every force entry is written before it is read.
   WT_CUDA(h, cudaMemsetAsync(err, 0, sizeof(unsigned), h->stream));
-  dispatch_steps(h, nsteps, path, part, fdev, err, kNaChunk);
+  dispatch_steps(h, nsteps, path, part, fdev, err, nullptr, kNaChunk);
   WT_CUDA(h, cudaGetLastError());
   double last[3] = {0, 0, 0};
   unsigned errw = 0;

@@ -34,23 +34,32 @@ struct wt_lattice {
   // per-step force reduction: one partial per 32-cell segment holding a near-wall cell
   long long nsegs = 0;           // 32-cell segments of the lattice (seg_of)
   int* wslot = nullptr;          // per segment: partial slot or -1
+  uint8_t* segmark = nullptr;    // per segment: 1 if it holds a near-wall cell
+  int* slot_scan = nullptr;      // scan workspace of launch_slots; the last entry is the slot count
   int nslots = 0;                // segments with a slot
   int part_cap = 0;              // slots that fit in `part` (per step of a chunk)
   double* part = nullptr;
-  double* forces_dev = nullptr;
-  double* forces_host = nullptr; // pinned
-  int forces_cap = 0;            // steps that fit in forces_dev / forces_host
-  unsigned* err_dev = nullptr;
-  unsigned* err_host = nullptr;  // pinned
+  double* forces_host = nullptr; // pinned; the reduction writes it directly
+  int forces_cap = 0;            // steps that fit in forces_host
+  unsigned* err_dev = nullptr;   // zero between calls
+  unsigned* err_host = nullptr;  // pinned, likewise written by the device
+  void* stage = nullptr;         // pinned staging of small view and sample calls
+  size_t stage_bytes = 0;
   double* sfrac = nullptr;       // partial bounce-back solid fraction on sbox (device), or null
+  double* sfrac_buf = nullptr;   // its memory, kept until the lattice goes
+  size_t sfrac_cap = 0;
   void* adj_pool = nullptr;      // device memory a wt_adjoint run with keep left for the next
   size_t adj_pool_bytes = 0;
   int sbox[6] = {0, 0, 0, 0, 0, 0};
-  // voxelize statistics scratch
+  // voxelize statistics scratch, one block read back by one copy
+  unsigned char* vstats = nullptr;
+  size_t vstats_bytes = 0;
+  int* counters = nullptr;       // [0] body cells, [1] wall velocity seen
+  int* low = nullptr;            // nx*nz lowest body cell per column
   uint8_t* col = nullptr;        // ny*nz frontal projection
   uint8_t* plan = nullptr;       // nx*nz planform projection
-  int* low = nullptr;            // nx*nz lowest body cell per column
-  int* counters = nullptr;       // [0] body cells, [1] wall velocity seen
+  void* vox_in = nullptr;        // the device copy of voxelize's mask or grid, kept while small
+  size_t vox_in_bytes = 0;
   // host-side state
   wt_params p{};
   wt_body_stats stats{};
@@ -105,13 +114,22 @@ cudaError_t configure_step_kernels(int nx, int storage);
 cudaError_t preload_step_kernels();
 cudaError_t preload_exact_step_kernels();
 
-// Deterministic per-step sum of the warp partials: out[3*s..3*s+2].
+// Deterministic per-step sum of the warp partials: out[3*s..3*s+2], device or
+// pinned host memory. With err_out the error word err is moved there and
+// zeroed (by the last launch of a call).
 void launch_force_reduce(const double* part, unsigned nslots, int nsteps, double* out,
-                         cudaStream_t s);
+                         unsigned* err, unsigned* err_out, cudaStream_t s);
 
-// mark[s] = 1 for every 32-cell segment s holding a near-wall cell.
-void launch_mark_segments(const uint8_t* flags, int nx, int ny, int nz, uint8_t* mark,
-                          cudaStream_t s);
+// Pinned staging of at least `bytes` bytes, which kernels read and write in
+// place of copies; null beyond kStageMax or when none is to be had.
+constexpr size_t kStageMax = 4u << 20;
+void* stage(wt_lattice* h, size_t bytes);
+
+// Number the 32-cell segments that carry a force partial (those with a near-wall
+// cell, segmark, and those that touch the solid-fraction box) in ascending
+// order: wslot, and their count in slot_scan[slot_scan_ints(h) - 1].
+int slot_scan_ints(const wt_lattice* h);
+void launch_slots(wt_lattice* h);
 
 // Equilibrium initialisation of both buffers and the fields:
 // mode 0 = reset(), mode 1 = reset() + seeded noise.

@@ -11,6 +11,7 @@
 //
 // Compiled without multiply-add contraction, in float64 like the reference.
 #include <math.h>
+#include <string.h>
 
 #include <cmath>
 
@@ -143,6 +144,15 @@ int wt_slice(wt_lattice* h, int plane, int k, int field, float* out, size_t len)
   if (k < 0 || k >= depth) return view_fail(h, WT_ERR_ARG, "plane index out of range");
   const size_t cells = (size_t)h->nx * (plane == 0 ? h->ny : h->nz);
   if (!out || len != cells) return view_fail(h, WT_ERR_ARG, "out must hold nx * (ny or nz) floats");
+  if (float* p = (float*)wt::stage(h, sizeof(float) * cells)) {   // written in place, pinned
+    k_slice<<<(unsigned)((cells + 255) / 256), 256, 0, h->stream>>>(view_of(h), plane, k, field, p);
+    h->launches++;
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return view_fail(h, WT_ERR_CUDA, "slice failed");
+    memcpy(out, p, sizeof(float) * cells);
+    return WT_OK;
+  }
   float* d = nullptr;
   if (cudaMalloc(&d, sizeof(float) * cells) != cudaSuccess)
     return view_fail(h, WT_ERR_OOM, "slice buffer");
@@ -160,8 +170,24 @@ int wt_advect(wt_lattice* h, double* xyz, int n, double kstep, uint8_t* expired,
   if (n < 0 || (n > 0 && !xyz) || !std::isfinite(kstep))
     return view_fail(h, WT_ERR_ARG, "bad particles or step");
   if (n == 0) return WT_OK;
-  unsigned char* d = nullptr;
   const size_t bytes = sizeof(double) * 3 * (size_t)n + (size_t)n + sizeof(float) * (size_t)n + 16;
+  if (double* p = (double*)wt::stage(h, bytes)) {
+    // a few thousand particles: the kernel works on them in pinned host memory,
+    // instead of one copy in and three out around it
+    float* sp = (float*)(p + 3 * (size_t)n);
+    uint8_t* ex = (uint8_t*)(sp + n);
+    memcpy(p, xyz, sizeof(double) * 3 * (size_t)n);
+    k_advect<<<(unsigned)((n + 63) / 64), 64, 0, h->stream>>>(view_of(h), p, n, kstep, ex, sp);
+    h->launches++;
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return view_fail(h, WT_ERR_CUDA, "advect failed");
+    memcpy(xyz, p, sizeof(double) * 3 * (size_t)n);
+    if (expired) memcpy(expired, ex, (size_t)n);
+    if (speed) memcpy(speed, sp, sizeof(float) * (size_t)n);
+    return WT_OK;
+  }
+  unsigned char* d = nullptr;
   if (cudaMalloc(&d, bytes) != cudaSuccess) return view_fail(h, WT_ERR_OOM, "particle buffer");
   double* dxyz = (double*)d;
   float* dsp = (float*)(d + sizeof(double) * 3 * (size_t)n);
