@@ -327,6 +327,18 @@ int wt_state_size(const wt_lattice* h, size_t* bytes);
 int wt_get_state(wt_lattice* h, void* out, size_t bytes);
 int wt_set_state(wt_lattice* h, const void* in, size_t bytes);
 
+/* The same state kept on the device (no reference counterpart): a snapshot costs
+ * device memory of the state's size and a copy at memory speed, where
+ * wt_get_state moves the state to the host. A snapshot is restored into the
+ * lattice it was taken from or one of the same device, dimensions and storage.
+ * wt_snapshot_create returns WT_ERR_OOM when there is no room for it.
+ * wt_snapshot_free: with keep, up to two blocks stay in the lattice h for its next
+ * snapshots (until wt_destroy); h may be NULL. */
+typedef struct wt_snapshot wt_snapshot;
+int wt_snapshot_create(wt_lattice* h, wt_snapshot** out);
+int wt_snapshot_restore(wt_lattice* h, const wt_snapshot* s);
+int wt_snapshot_free(wt_lattice* h, wt_snapshot* s, int keep);
+
 /* LBM.sample(x, y, z, out) — js/lbm.js:515-539 — for npts points (xyz holds
  * 3*npts doubles, out receives 3*npts doubles). Trilinear at cell centres,
  * (u0,0,0) outside the half-cell margin. */

@@ -146,6 +146,9 @@ SIGNATURES = {
     "wt_state_size": [_P, C.POINTER(C.c_size_t)],
     "wt_get_state": [_P, C.c_void_p, C.c_size_t],
     "wt_set_state": [_P, C.c_void_p, C.c_size_t],
+    "wt_snapshot_create": [_P, C.POINTER(_P)],
+    "wt_snapshot_restore": [_P, _P],
+    "wt_snapshot_free": [_P, _P, C.c_int],
     "wt_sample": [_P, _D, C.c_int, _D],
     "wt_is_solid": [_P, C.c_double, C.c_double, C.c_double, _I],
     "wt_get_stream": [_P, C.POINTER(_P)],

@@ -4,7 +4,7 @@
 of `nsteps` steps of lattice `sim` from its current state, with the solid
 fraction `s` (a [z][y][x] tensor over `box`) applied by partial bounce-back.
 Its backward calls wt_adjoint through the C ABI from the same starting state
-(saved with wt_get_state), so autograd sees the hand-written discrete adjoint
+(kept on the device, wt_snapshot_create), so autograd sees the hand-written discrete adjoint
 of the fused CUDA step; nothing is differentiated by torch itself.
 """
 from __future__ import annotations
@@ -12,7 +12,38 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from ._lib import WT_ERR_OOM, WTError
 from .lbm import LBM
+
+
+class _Start:
+    """The lattice's state at one moment: a device snapshot, or where there is no
+    device memory for one, the host copy of wt_get_state."""
+
+    def __init__(self, sim: LBM, keep: bool):
+        self.sim, self.keep, self.snap, self.blob = sim, keep, None, None
+        try:
+            self.snap = sim.snapshot()
+        except WTError as e:
+            if e.code != WT_ERR_OOM:
+                raise
+            self.blob = sim.get_state()
+
+    def restore(self) -> None:
+        if self.snap is not None:
+            self.sim.restore(self.snap)
+        else:
+            self.sim.set_state(self.blob)
+
+    def close(self) -> None:
+        if self.snap is not None:
+            self.snap.close(self.keep)
+
+    def __del__(self):
+        try:
+            self.close()
+        except Exception:
+            pass
 
 
 class DragFn(torch.autograd.Function):
@@ -21,7 +52,7 @@ class DragFn(torch.autograd.Function):
                 component: int = 0, checkpoint: int = 0, keep: bool = False):
         sv = s.detach().to("cpu", torch.float64).numpy()
         sim.set_solid_fraction(box, sv)
-        start = sim.get_state()
+        start = _Start(sim, bool(keep)) if ctx.needs_input_grad[0] else None
         f = sim.step_forces(int(nsteps))
         J = float(f[-int(window):, component].mean())
         ctx.sim, ctx.box, ctx.start, ctx.sv = sim, box, start, sv
@@ -32,11 +63,12 @@ class DragFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gJ: torch.Tensor):
         sim = ctx.sim
-        end = sim.get_state()
-        sim.set_state(ctx.start)
+        end = _Start(sim, ctx.cfg[-1])
+        ctx.start.restore()
         sim.set_solid_fraction(ctx.box, ctx.sv)
         _, g, _ = sim.adjoint(*ctx.cfg)
-        sim.set_state(end)   # the lattice stays where the forward pass left it
+        end.restore()   # the lattice stays where the forward pass left it
+        end.close()
         dtype, device = ctx.s_meta
         grad = torch.from_numpy(np.ascontiguousarray(g)).to(device=device, dtype=dtype)
         return gJ.to(dtype) * grad, None, None, None, None, None, None, None

@@ -4,6 +4,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -12,6 +13,12 @@
 namespace {
 
 thread_local std::string g_create_error;
+
+// Numbers every occupancy any lattice is given (wt_lattice::occupancy).
+uint64_t next_occupancy() {
+  static std::atomic<uint64_t> last{0};
+  return ++last;
+}
 
 constexpr int kChunk = 32;         // steps whose force partials are reduced together
 constexpr uint32_t kStateMagic = 0x57545354u;  // "WTST"
@@ -79,6 +86,8 @@ void free_all(wt_lattice* h) {
   if (h->aux) cudaStreamDestroy(h->aux);
   if (h->adj_pool) cudaFree(h->adj_pool);
   h->adj_pool = nullptr;
+  for (void* m : h->snap_mem)
+    if (m) cudaFree(m);
 }
 
 int check_params(const wt_params* p) {
@@ -557,6 +566,7 @@ int voxelize_finish(wt_lattice* h, int ground, double road_vel) {
 }
 
 int voxelize_start(wt_lattice* h, int ground, double road_vel) {
+  h->occupancy = next_occupancy();
   wt::launch_clear_obj(h);
   wt::launch_floor(h, ground, road_vel);
   WT_CUDA(h, cudaMemsetAsync(h->vstats, 0, h->vstats_bytes, h->stream));
@@ -876,6 +886,46 @@ struct StateHeader {
   wt_body_stats stats;
 };
 
+StateHeader state_header(const wt_lattice* h) {
+  StateHeader hd{};
+  hd.magic = kStateMagic;
+  hd.nx = h->nx; hd.ny = h->ny; hd.nz = h->nz; hd.storage = h->storage; hd.parity = h->parity;
+  hd.steps = h->steps;
+  memcpy(hd.force, h->force, sizeof(hd.force));
+  hd.params = h->p;
+  hd.stats = h->stats;
+  return hd;
+}
+
+void apply_header(wt_lattice* h, const StateHeader& hd) {
+  h->parity = hd.parity & 1;
+  h->steps = hd.steps;
+  memcpy(h->force, hd.force, sizeof(hd.force));
+  h->p = hd.params;
+  h->stats = hd.stats;
+}
+
+// Copies between a lattice and a snapshot's block (populations A and B, flags,
+// fields), out of the lattice or into it, with or without the flags; waits.
+cudaError_t snapshot_copy(wt_lattice* h, unsigned char* mem, size_t pop, size_t nb, size_t fb,
+                          bool out, bool flags) {
+  cudaError_t e = cudaSuccess;
+  auto one = [&](void* lat, size_t bytes, size_t room) {
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(out ? (void*)mem : lat, out ? lat : (void*)mem, bytes,
+                          cudaMemcpyDeviceToDevice, h->stream);
+    mem += room;
+  };
+  one(h->buf[0], (size_t)h->n * 19 * h->elem, pop);
+  one(h->buf[1], (size_t)h->n * 19 * h->elem, pop);
+  if (flags) one(h->flags, (size_t)h->n, nb);
+  else mem += nb;
+  for (float* p : {h->ux, h->uy, h->uz, h->rho, h->uwx, h->uwy, h->uwz})
+    one(p, sizeof(float) * (size_t)h->n, fb);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  return e;
+}
+
 size_t state_bytes(const wt_lattice* h) {
   return sizeof(StateHeader) + 2 * (size_t)h->n * 19 * h->elem + (size_t)h->n +
          7 * sizeof(float) * (size_t)h->n;
@@ -891,13 +941,7 @@ int wt_state_size(const wt_lattice* h, size_t* bytes) {
 int wt_get_state(wt_lattice* h, void* out, size_t bytes) {
   if (!h || !out) return WT_ERR_ARG;
   if (bytes != state_bytes(h)) return fail(h, WT_ERR_ARG, "state buffer has the wrong size");
-  StateHeader hd{};
-  hd.magic = kStateMagic;
-  hd.nx = h->nx; hd.ny = h->ny; hd.nz = h->nz; hd.storage = h->storage; hd.parity = h->parity;
-  hd.steps = h->steps;
-  memcpy(hd.force, h->force, sizeof(hd.force));
-  hd.params = h->p;
-  hd.stats = h->stats;
+  const StateHeader hd = state_header(h);
   char* o = (char*)out;
   memcpy(o, &hd, sizeof(hd));
   o += sizeof(hd);
@@ -934,14 +978,84 @@ int wt_set_state(wt_lattice* h, const void* in, size_t bytes) {
     o += fb;
   }
   WT_CUDA(h, cudaStreamSynchronize(h->stream));
-  h->parity = hd.parity & 1;
-  h->steps = hd.steps;
-  memcpy(h->force, hd.force, sizeof(hd.force));
-  h->p = hd.params;
-  h->stats = hd.stats;
+  apply_header(h, hd);
+  h->occupancy = next_occupancy();
   wt::launch_near(h);   // near flags and neighbour masks follow from the restored occupancy
   WT_CUDA(h, cudaStreamSynchronize(h->stream));
   return rebuild_slots(h);
+}
+
+// A state on the device: what wt_get_state copies out, in one device block.
+struct wt_snapshot {
+  StateHeader hd;
+  uint64_t occupancy;   // wt_lattice::occupancy at the time
+  int device;
+  size_t bytes;
+  unsigned char* mem;
+};
+
+int wt_snapshot_create(wt_lattice* h, wt_snapshot** out) {
+  if (!h) return WT_ERR_ARG;
+  if (!out) return fail(h, WT_ERR_ARG, "out is NULL");
+  *out = nullptr;
+  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t pop = up((size_t)h->n * 19 * h->elem), fb = up(sizeof(float) * (size_t)h->n),
+               nb = up((size_t)h->n), bytes = 2 * pop + nb + 7 * fb;
+  wt_snapshot* s = new wt_snapshot{state_header(h), h->occupancy, h->device, bytes, nullptr};
+  // a block that a freed snapshot left in the lattice, or a new one
+  for (void*& m : h->snap_mem)
+    if (m && !s->mem) {
+      s->mem = (unsigned char*)m;
+      m = nullptr;
+    }
+  if (!s->mem && cudaMalloc((void**)&s->mem, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    delete s;
+    return fail(h, WT_ERR_OOM, "cannot allocate a snapshot of " + std::to_string(bytes >> 20) + " MiB");
+  }
+  const cudaError_t e = snapshot_copy(h, s->mem, pop, nb, fb, true, true);
+  if (e != cudaSuccess) {
+    cudaFree(s->mem);
+    delete s;
+    return cuda_fail(h, e, "snapshot");
+  }
+  *out = s;
+  return WT_OK;
+}
+
+int wt_snapshot_restore(wt_lattice* h, const wt_snapshot* s) {
+  if (!h) return WT_ERR_ARG;
+  if (!s) return fail(h, WT_ERR_ARG, "snapshot is NULL");
+  const StateHeader& hd = s->hd;
+  if (hd.nx != h->nx || hd.ny != h->ny || hd.nz != h->nz || hd.storage != h->storage ||
+      s->device != h->device)
+    return fail(h, WT_ERR_ARG, "snapshot was taken from a different lattice");
+  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t pop = up((size_t)h->n * 19 * h->elem), fb = up(sizeof(float) * (size_t)h->n),
+               nb = up((size_t)h->n);
+  // the same occupancy: its flags, masks and slots are in place
+  const bool same = s->occupancy == h->occupancy;
+  const cudaError_t e = snapshot_copy(h, s->mem, pop, nb, fb, false, !same);
+  if (e != cudaSuccess) return cuda_fail(h, e, "snapshot restore");
+  apply_header(h, hd);
+  if (same) return WT_OK;
+  h->occupancy = s->occupancy;
+  wt::launch_near(h);
+  return rebuild_slots(h);
+}
+
+int wt_snapshot_free(wt_lattice* h, wt_snapshot* s, int keep) {
+  if (!s) return WT_OK;
+  if (h && keep && s->device == h->device && s->hd.nx == h->nx && s->hd.ny == h->ny &&
+      s->hd.nz == h->nz && s->hd.storage == h->storage)
+    for (void*& m : h->snap_mem)
+      if (!m && s->mem) {
+        m = s->mem;   // for the lattice's next snapshot
+        s->mem = nullptr;
+      }
+  if (s->mem) cudaFree(s->mem);
+  delete s;
+  return WT_OK;
 }
 
 int wt_sample(wt_lattice* h, const double* xyz, int npts, double* out) {

@@ -51,6 +51,8 @@ struct wt_lattice {
   void* adj_pool = nullptr;      // device memory a wt_adjoint run with keep left for the next
   size_t adj_pool_bytes = 0;
   int sbox[6] = {0, 0, 0, 0, 0, 0};
+  uint64_t occupancy = 0;        // changes with every change of the flags and wall velocities
+  void* snap_mem[2] = {nullptr, nullptr};   // blocks that freed snapshots left for the next ones
   // voxelize statistics scratch, one block read back by one copy
   unsigned char* vstats = nullptr;
   size_t vstats_bytes = 0;

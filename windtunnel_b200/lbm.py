@@ -451,6 +451,16 @@ class LBM:
         self._call(lib().wt_set_state, buf, len(blob))
         self._fields_at = -1
 
+    def snapshot(self) -> "Snapshot":
+        """The state kept on the device: restore() it into this lattice or a like one."""
+        s = C.c_void_p()
+        self._call(lib().wt_snapshot_create, C.byref(s))
+        return Snapshot(self, s)
+
+    def restore(self, snap: "Snapshot") -> None:
+        self._call(lib().wt_snapshot_restore, snap._s)
+        self._fields_at = -1
+
     # ---- sampling (js/lbm.js:515-545) ------------------------------------------------------
     def sample(self, x: float, y: float, z: float, out=None):
         v = self.sample_points(np.array([[x, y, z]], np.float64))[0]
@@ -486,6 +496,27 @@ class LBM:
         c = C.c_int64()
         self._call(lib().wt_get_launch_count, C.byref(c))
         return c.value
+
+
+class Snapshot:
+    """A lattice's state in device memory (LBM.snapshot). close(keep=True) leaves
+    the memory in the lattice for its next snapshot."""
+
+    def __init__(self, sim: LBM, s: C.c_void_p):
+        self._sim = sim
+        self._s = s
+
+    def close(self, keep: bool = False) -> None:
+        if self._s is not None and self._s.value:
+            h = self._sim._h
+            lib().wt_snapshot_free(h if h.value else None, self._s, int(bool(keep)))
+        self._s = None
+
+    def __del__(self):
+        try:
+            self.close()
+        except Exception:
+            pass
 
 
 def _evaluate_inside(inside, X: np.ndarray, Y: np.ndarray, Z: np.ndarray) -> np.ndarray:
