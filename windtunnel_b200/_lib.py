@@ -149,6 +149,8 @@ SIGNATURES = {
     "wt_snapshot_create": [_P, C.POINTER(_P)],
     "wt_snapshot_restore": [_P, _P],
     "wt_snapshot_free": [_P, _P, C.c_int],
+    "wt_host_alloc": [C.c_size_t],
+    "wt_host_free": [_P],
     "wt_sample": [_P, _D, C.c_int, _D],
     "wt_is_solid": [_P, C.c_double, C.c_double, C.c_double, _I],
     "wt_get_stream": [_P, C.POINTER(_P)],
@@ -162,7 +164,8 @@ SIGNATURES = {
     "wt_slice": [_P, C.c_int, C.c_int, C.c_int, _F, C.c_size_t],
     "wt_advect": [_P, _D, C.c_int, C.c_double, _U8, _F],
 }
-_RESTYPES = {"wt_default_params": None, "wt_last_error": C.c_char_p,
+_RESTYPES = {"wt_default_params": None, "wt_host_alloc": C.c_void_p, "wt_host_free": None,
+             "wt_last_error": C.c_char_p,
              "wt_voxel_last_error": C.c_char_p}
 
 _lib: C.CDLL | None = None

@@ -35,6 +35,7 @@ UNITS = {
     "wt_api.cu": [],
     "wt_voxel.cu": ["--fmad=false"],
     "wt_view.cu": ["--fmad=false"],
+    "wt_host.cu": [],
 }
 
 

@@ -54,6 +54,43 @@ def _box6(box) -> np.ndarray:
     return np.ascontiguousarray(v, dtype=np.float64)
 
 
+class _HostBlock:
+    """Pooled page-locked memory as a numpy buffer; back to the pool with its last array."""
+
+    __slots__ = ("ptr", "__array_interface__")
+
+    def __init__(self, ptr: int, count: int, dtype):
+        self.ptr = ptr
+        self.__array_interface__ = {"version": 3, "shape": (count,), "data": (ptr, False),
+                                    "typestr": np.dtype(dtype).str}
+
+    def __del__(self):
+        try:
+            lib().wt_host_free(self.ptr)
+        except Exception:
+            pass
+
+
+_asked: set = set()   # result sizes that were asked for before
+
+
+def _results(count: int, dtype, arrays: int = 1) -> list[np.ndarray]:
+    """Arrays for results of a device call: from the page-locked pool where a size
+    is asked for again, so that a program that reads a large field once does not
+    pay for page-locking, else (and for small or refused sizes) plain ones."""
+    size = count * np.dtype(dtype).itemsize
+    known = size in _asked
+    if not known and size >= 1 << 20:
+        if len(_asked) >= 64:
+            _asked.clear()
+        _asked.add(size)
+    out = []
+    for _ in range(arrays):
+        p = lib().wt_host_alloc(size) if known else None
+        out.append(np.asarray(_HostBlock(p, count, dtype)) if p else np.empty(count, dtype))
+    return out
+
+
 class LBM:
     """D3Q19 lattice on the current CUDA device (the reference `new LBM(nx, ny, nz)`)."""
 
@@ -318,7 +355,7 @@ class LBM:
     # ---- fields (js/lbm.js:82-88) ------------------------------------------------------
     def fields(self) -> tuple[np.ndarray, np.ndarray, np.ndarray, np.ndarray]:
         """(ux, uy, uz, rho), each a float32 array of n cells, fresh from the device."""
-        a = [np.empty(self.n, np.float32) for _ in range(4)]
+        a = _results(self.n, np.float32, 4)
         self._call(lib().wt_get_fields, *[x.ctypes.data_as(C.POINTER(C.c_float)) for x in a])
         return tuple(a)
 
@@ -347,13 +384,13 @@ class LBM:
 
     @property
     def solid(self) -> np.ndarray:
-        out = np.empty(self.n, np.uint8)
+        out = _results(self.n, np.uint8)[0]
         self._call(lib().wt_get_solid, out.ctypes.data_as(C.POINTER(C.c_uint8)))
         return out
 
     @property
     def near(self) -> np.ndarray:
-        out = np.empty(self.n, np.uint8)
+        out = _results(self.n, np.uint8)[0]
         self._call(lib().wt_get_near, out.ctypes.data_as(C.POINTER(C.c_uint8)))
         return out
 
@@ -364,7 +401,7 @@ class LBM:
         if dtype == "raw":
             code = STORAGE[self.storage]
         npd = _STORE_DTYPE[code]
-        out = np.empty(19 * self.n, npd)
+        out = _results(19 * self.n, npd)[0]
         self._call(lib().wt_get_populations, W.WT_BUF_F if which == "f" else W.WT_BUF_G, code,
                    out.ctypes.data, out.nbytes)
         return out.reshape(19, self.n)
@@ -442,13 +479,16 @@ class LBM:
     def get_state(self) -> bytes:
         size = C.c_size_t()
         self._call(lib().wt_state_size, C.byref(size))
-        buf = (C.c_char * size.value)()
-        self._call(lib().wt_get_state, buf, size.value)
-        return bytes(buf)
+        # the bytes object's own memory, filled before anyone sees it
+        new = C.pythonapi.PyBytes_FromStringAndSize
+        new.restype, new.argtypes = C.py_object, [C.c_void_p, C.c_ssize_t]
+        blob = new(None, size.value)
+        self._call(lib().wt_get_state, C.cast(C.c_char_p(blob), C.c_void_p), size.value)
+        return blob
 
     def set_state(self, blob: bytes) -> None:
-        buf = C.create_string_buffer(blob, len(blob))
-        self._call(lib().wt_set_state, buf, len(blob))
+        data = blob if isinstance(blob, bytes) else bytes(blob)
+        self._call(lib().wt_set_state, C.cast(C.c_char_p(data), C.c_void_p), len(data))
         self._fields_at = -1
 
     def snapshot(self) -> "Snapshot":
