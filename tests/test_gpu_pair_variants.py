@@ -47,6 +47,38 @@ def test_auto_float32_agrees_with_direct(wt_lib, dims, moving, side_bc):
     assert np.abs(ga - gb).max() <= 1e-6
 
 
+@pytest.mark.parametrize("dims", [(17, 9, 9), (33, 9, 8), (65, 9, 9), (257, 7, 6)])
+@pytest.mark.parametrize("side_bc", ["eq", "freeslip"])
+@pytest.mark.parametrize("les,trt", [(True, True), (True, False), (False, True)])
+def test_odd_width_is_the_lean_kernel(wt_lib, dims, side_bc, les, trt):
+    """The odd-width form performs the lean kernel's operations: the same bits."""
+    _same_bits(dims, "lean", side_bc, les, trt, 0.0)
+
+
+@pytest.mark.parametrize("dims", [(17, 9, 9), (34, 9, 8), (65, 9, 9), (160, 9, 8), (256, 8, 7)])
+@pytest.mark.parametrize("side_bc", ["eq", "freeslip"])
+@pytest.mark.parametrize("les,trt", [(True, True), (True, False), (False, True)])
+def test_moving_walls_are_the_direct_kernel(wt_lib, dims, side_bc, les, trt):
+    """The moving-wall form performs the direct kernel's operations: the same bits."""
+    _same_bits(dims, "direct", side_bc, les, trt, 0.03)
+
+
+def _same_bits(dims, kernel, side_bc, les, trt, road):
+    from windtunnel_b200 import LBM
+    nx, ny, nz = dims
+    body = (nx - 4.5, ny / 2, nz / 2, 2.6)
+    out = []
+    for k in (kernel, "auto"):
+        s = LBM(*dims, kernel=k, side_bc=side_bc)
+        apply_case(s, sphere=body, side_bc=side_bc, ground=True, roadVel=road, les=les, trt=trt,
+                   tau=0.53, wallVel=spinning_sphere_wallvel(*body[:3], 0.01) if road else None)
+        f = s.step_forces(12)
+        out.append([f, s.populations("f", "raw"), s.populations("g", "raw"), *s.fields()])
+    assert np.abs(out[0][0] - out[1][0]).max() <= 1e-12 * np.abs(out[0][0]).max()
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("dims", [(33, 9, 8), (34, 9, 8), (97, 12, 11), (160, 9, 8)])
 @pytest.mark.parametrize("moving", [False, True])
 def test_exact_form_is_the_oracle_across_row_ends(wt_lib, oracle_lib, dims, moving):

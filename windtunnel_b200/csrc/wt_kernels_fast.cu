@@ -54,8 +54,11 @@ using PairKernel = void (*)(StepArgs<S>);
 template <class S>
 PairKernel<S> pair_kernel(bool sr, int mode) {
   if constexpr (sizeof(S) == 2) {
-    if (sr) return mode & PAIR_ROWS ? k_step_pair<S, true, PAIR_ROWS> : k_step_pair<S, true, 0>;
-    return mode & PAIR_ROWS ? k_step_pair<S, false, PAIR_ROWS> : k_step_pair<S, false, 0>;
+    switch (mode) {
+      case PAIR_ROWS: return sr ? k_step_pair<S, true, PAIR_ROWS> : k_step_pair<S, false, PAIR_ROWS>;
+      case PAIR_PBB: return k_step_pair<S, false, PAIR_PBB>;
+      default: return sr ? k_step_pair<S, true, 0> : k_step_pair<S, false, 0>;
+    }
   } else {
     switch (mode) {
       case PAIR_ODD: return k_step_pair<S, false, PAIR_ODD>;
@@ -70,17 +73,15 @@ PairKernel<S> pair_kernel(bool sr, int mode) {
   }
 }
 
-// Every variant, for the preload loop below.
-constexpr int kPairModes[] = {0, PAIR_ROWS, PAIR_ODD, PAIR_MOV, PAIR_ROWS | PAIR_MOV,
-                              PAIR_ODD | PAIR_MOV};
+// Every variant a wt_step_noalloc call can launch, for the preload loop below.
 template <class F>
 cudaError_t each_pair_kernel(F f) {
   cudaError_t e = cudaSuccess;
-  for (int m : kPairModes) {
+  for (int m : {0, (int)PAIR_ROWS, (int)PAIR_ODD, (int)PAIR_MOV, PAIR_ROWS | PAIR_MOV,
+                PAIR_ODD | PAIR_MOV}) {
     if (e == cudaSuccess) e = f((const void*)pair_kernel<float>(false, m));
     for (bool sr : {false, true})
-      if (e == cudaSuccess && !(m & (PAIR_ODD | PAIR_MOV)))
-        e = f((const void*)pair_kernel<__half>(sr, m));
+      if (e == cudaSuccess && !(m & (PAIR_ODD | PAIR_MOV))) e = f((const void*)pair_kernel<__half>(sr, m));
   }
   return e;
 }
@@ -97,15 +98,22 @@ void launch_pair_f32(const StepArgs<float>& a, dim3, bool, cudaStream_t s) { lau
 
 // ---- partial bounce-back and adjoint (float32 arithmetic) -------------------------
 
-// The float32 partial-bounce-back step runs the pair kernel (PAIR_PBB), except
-// with moving walls or buffers of 2^31 bytes or more.
+// The partial-bounce-back step runs the pair kernel (PAIR_PBB), except with
+// moving walls, buffers of 2^31 bytes or more, and in half storage an odd nx.
+template <class S>
+bool pbb_pair_ok(const StepArgs<S>& a) {
+  return !a.mov && 19 * a.n * (long long)sizeof(S) < (1LL << 31) &&
+         (sizeof(S) == 4 || a.nx % 2 == 0);
+}
+
 void launch_pbb_f32_fast(const StepArgs<float>& a, dim3 grid, bool wide, cudaStream_t s) {
-  if (!a.mov && 19 * a.n * (long long)sizeof(float) < (1LL << 31)) return launch_pair(a, s);
+  if (pbb_pair_ok(a)) return launch_pair(a, s);
   if (wide) launch_pdl(k_step_pbb<float, false, long long>, grid, dim3(STEP_BX), s, a);
   else launch_pdl(k_step_pbb<float, false, int>, grid, dim3(STEP_BX), s, a);
 }
 
 void launch_pbb_f16_fast(const StepArgs<__half>& a, dim3 grid, bool wide, cudaStream_t s) {
+  if (pbb_pair_ok(a)) return launch_pair(a, s);
   if (wide) launch_pdl(k_step_pbb<__half, false, long long>, grid, dim3(STEP_BX), s, a);
   else launch_pdl(k_step_pbb<__half, false, int>, grid, dim3(STEP_BX), s, a);
 }

@@ -46,14 +46,15 @@
 namespace wt {
 
 // Threads per block and the resident blocks per SM the register budget is set
-// for, the fastest measured on B200 (launched with programmatic dependent
-// launch): 128 threads for both storages; half storage 7 blocks (72 registers,
-// 28 warps; 80 registers at 24 warps lose 3%; 64-thread blocks 0.9% and 32-thread
-// blocks 8% slower), float32 storage 6 blocks (80 registers, no spills, 24
-// warps; 64-thread blocks 1.5% slower); with an odd nx or moving walls 5, where 6
-// spill (193x85x91: 39.8 against 57.0 us a step; 160x80x80 over a road: 31.0 against
-// 32.9, and 33.6 with 4, in plane order); with partial bounce-back 4 (128x64x64, a
-// 32^3 box: 12.9 us a step, 5 blocks 14.4, 6 22.4; the one-cell kernel 18.5).
+// for (pair_min_blocks), the fastest measured on B200 (launched with programmatic
+// dependent launch): 128 threads for both storages; half storage 7 blocks (72
+// registers, 28 warps; 80 registers at 24 warps lose 3%; 64-thread blocks 0.9%
+// and 32-thread blocks 8% slower), float32 storage 6 blocks (80 registers, no
+// spills, 24 warps; 64-thread blocks 1.5% slower). The variants' figures,
+// microseconds a step by number of blocks: odd nx (193x85x91) 4: 41.3, 5: 41.9, 6:
+// 54; moving walls (160x80x80 over a road) 4: 32.1, 5: 29.3, 6: 32.0; partial
+// bounce-back float32 (128x64x64, a 32^3 box) 3: 15.3, 4: 13.3, 5: 14.5, half storage
+// (384x160x160, a 64^3 box) 4: 239, 5: 244, 6: 266.
 constexpr int PAIR_BX = 128;
 
 // Variants of the pair kernel. ODD: an odd nx (float32 storage only): pairs
@@ -64,19 +65,34 @@ constexpr int PAIR_BX = 128;
 // of 256: each block is an x-segment of one row (grid x, y, z); else the pairs
 // of a plane are numbered along x, then y, across the rows' ends, so that
 // every lane has a pair whatever nx is, for one division per thread. PBB: a
-// partial bounce-back field (wt_pbb.cuh, float32 storage only): the blend of a
-// box cell's outputs with its reversed inputs, and its force.
-// Measured on B200, microseconds a step, one-cell kernels before / pair kernel:
-// 193x85x91 float32 46.3 / 39.8 (ODD against lean); 160x80x80 float32 over a rolling
-// road 40.3 / 28.7 (MOV against direct). Pairs across row ends against one row
-// per block: 64x32x32 float32 8.2 / 6.7 us (three of a block's four warps had
-// nothing to do); on 256x128x128 and 512x192x192 one row per block is 1-2% faster
-// for half storage.
+// partial bounce-back field (wt_pbb.cuh): the blend of a box cell's outputs with
+// its reversed inputs, and its force.
+// Measured on B200, microseconds a step, one-cell kernel / pair kernel: 193x85x91
+// float32 46.3 / 41.3 (ODD against lean); 160x80x80 float32 over a rolling road
+// 40.3 / 29.3 (MOV against direct); PBB float32 18.5 / 13.3, half storage 289 / 239. Pairs
+// across row ends against one row per block: 64x32x32 float32 8.2 / 6.7 us (three of
+// a block's four warps had nothing to do); on 256x128x128 and 512x192x192 one row
+// per block is 1-2% faster for half storage.
 enum : int { PAIR_ODD = 1, PAIR_MOV = 2, PAIR_ROWS = 4, PAIR_PBB = 8 };
+
+// Whose arithmetic a variant computes. The variants that stand for a one-cell
+// kernel perform that kernel's operations in its order, two cells at once
+// (packed fused multiply-adds where the compiler contracts the scalar
+// expressions), so that results are the same bit for bit whichever kernel a
+// lattice's width, walls or storage select: lean (collide_x2) for an odd nx,
+// direct (collide_fast) for moving walls, k_step_pbb (cell_fw_pairs) for
+// partial bounce-back. Tests hold them to that.
+enum : int { ARITH_OWN, ARITH_LEAN, ARITH_DIRECT, ARITH_PBB };
+constexpr int pair_arith(int mode) {
+  return mode & PAIR_PBB ? ARITH_PBB
+                         : (mode & PAIR_MOV ? ARITH_DIRECT : (mode & PAIR_ODD ? ARITH_LEAN : ARITH_OWN));
+}
 
 template <class S>
 constexpr int pair_min_blocks(int mode) {
-  return sizeof(S) == 2 ? 7 : (mode & PAIR_PBB ? 4 : (mode & (PAIR_MOV | PAIR_ODD) ? 5 : 6));
+  if (mode & PAIR_PBB) return 4;
+  if (sizeof(S) == 2) return 7;
+  return mode & PAIR_MOV ? 5 : (mode & PAIR_ODD ? 4 : 6);
 }
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
@@ -135,19 +151,25 @@ struct PairIO<__half> {
   struct Raw { uint32_t w, h; };
   template <int dx, bool ODD>
   __device__ __forceinline__ static Raw load(const char* p) {
-    if constexpr (dx == 0) return Raw{ld32(p), 0u};
+    if constexpr (ODD) return Raw{ld16(p), ld16(p + 2)};
+    else if constexpr (dx == 0) return Raw{ld32(p), 0u};
     else if constexpr (dx == 1) return Raw{ld32(p + 2), ld16(p)};
     else return Raw{ld32(p - 2), ld16(p + 2)};
   }
-  template <int dx>
+  template <int dx, bool ODD>
   __device__ __forceinline__ static W join(const Raw& r) {
-    if constexpr (dx == 0) return r.w;
+    if constexpr (ODD) return prmt(r.w, r.h, 0x5410u);
+    else if constexpr (dx == 0) return r.w;
     else if constexpr (dx == 1) return prmt(r.h, r.w, 0x5410u);
     else return prmt(r.w, r.h, 0x5432u);
   }
+  __device__ __forceinline__ static void opaque(W& w) { asm volatile("" : "+r"(w)); }
   __device__ __forceinline__ static f2 to_f2(W w) { return h2f(w); }
   __device__ __forceinline__ static W pack(f2 g) { return f2h(g); }
   __device__ __forceinline__ static W pack_sr(f2 g, uint32_t r) { return f2h_sr(g, r); }
+  // words of the high / low halves of two words
+  __device__ __forceinline__ static W highs(W x, W y) { return prmt(x, y, 0x7632u); }
+  __device__ __forceinline__ static W lows(W x, W y) { return prmt(x, y, 0x5410u); }
   __device__ __forceinline__ static W eq(const StepArgs<__half>& a, int q) { return a.eq2[q]; }
   __device__ __forceinline__ static W fix(W v, W e, bool inlet, bool outlet) {
     return prmt(v, e, inlet ? 0x3254u : (outlet ? 0x1010u : 0x3210u));
@@ -174,11 +196,14 @@ struct PairIO<float> {
     if constexpr (dx == 0 && !ODD) return *reinterpret_cast<const float2*>(p);
     else return make_float2(*reinterpret_cast<const float*>(p), *reinterpret_cast<const float*>(p + 4));
   }
-  template <int dx>
+  template <int dx, bool ODD>
   __device__ __forceinline__ static W join(const Raw& r) { return r; }
+  __device__ __forceinline__ static void opaque(W& w) { asm volatile("" : "+f"(w.x), "+f"(w.y)); }
   __device__ __forceinline__ static f2 to_f2(W w) { return w; }
   __device__ __forceinline__ static W pack(f2 g) { return g; }
   __device__ __forceinline__ static W pack_sr(f2 g, uint32_t) { return g; }
+  __device__ __forceinline__ static W highs(W x, W y) { return make_float2(x.y, y.y); }
+  __device__ __forceinline__ static W lows(W x, W y) { return make_float2(x.x, y.x); }
   __device__ __forceinline__ static W eq(const StepArgs<float>& a, int q) {
     return make_float2(a.eq[q], a.eq[q]);
   }
@@ -416,7 +441,7 @@ __device__ __forceinline__ PairCells pair_cells(uint32_t fl, int x0, int nx) {
 // (0 for cells that are not computed), F their blend's force before the factor sf.
 template <class S, bool SR, int MODE, bool BLEND>
 __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
-                                                   const typename PairIO<S>::W (&w)[Q],
+                                                   typename PairIO<S>::W (&w)[Q],
                                                    long long i0, const PairCells& cells,
                                                    f2 sf, f2 (&F)[3]) {
   using IO = PairIO<S>;
@@ -432,33 +457,18 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     return *reinterpret_cast<R*>(Gb + a.dstb[q] + sizeof(R) * L);
   };
   // ---- pass 1: moments --------------------------------------------------
-  // ODD, MOV and PBB: the moments are summed in trees, the momentum j = r u is
-  // carried through the update, and the relaxation is added to f instead of
-  // scaling f by a rounded 1 - om, so that a step conserves mass and momentum to
-  // the rounding of its sums. With the other variants' arithmetic (kept as it
-  // is: their results are compared from release to release) the error of u
-  // against float64 after 100 steps was 1.3 to 2 times that of the one-cell
-  // kernels these stand for; so it is 0.3 to 0.6 of theirs (B200, 160x80x80
-  // over a road: uz 1.2e-6 against 1.9e-6; 193x85x91: 7.4e-7 against 1.4e-6).
-  constexpr bool PBB = (MODE & PAIR_PBB) != 0;
-  constexpr bool MOM = ODD || MOV || PBB;
+  constexpr int AR = pair_arith(MODE);
+  constexpr bool REF = AR != ARITH_OWN;
+  auto sum = [&](int q) { return padd(IO::to_f2(w[q]), IO::to_f2(w[q + 1])); };
+  auto dif = [&](int q) { return psub(IO::to_f2(w[q]), IO::to_f2(w[q + 1])); };
   f2 dr, jx, jy, jz, pxx, pyy, pzz, pxy, pxz, pyz;
-  if constexpr (MOM) {
-    auto sum = [&](int q) { return padd(IO::to_f2(w[q]), IO::to_f2(w[q + 1])); };
-    auto dif = [&](int q) { return psub(IO::to_f2(w[q]), IO::to_f2(w[q + 1])); };
-    const f2 s1 = sum(1), s3 = sum(3), s5 = sum(5);
-    const f2 faces = padd(padd(IO::to_f2(w[0]), s1), padd(s3, s5));
-    f2 s = sum(7), t = sum(9), d = dif(7), e = dif(9);
-    const f2 xy = padd(s, t);
-    pxy = psub(s, t); jx = padd(dif(1), padd(d, e)); jy = padd(dif(3), psub(d, e));
-    s = sum(11); t = sum(13); d = dif(11); e = dif(13);
-    const f2 xz = padd(s, t);
-    pxz = psub(s, t); jx = padd(jx, padd(d, e)); jz = padd(dif(5), psub(d, e));
-    s = sum(15); t = sum(17); d = dif(15); e = dif(17);
-    const f2 yz = padd(s, t);
-    pyz = psub(s, t); jy = padd(jy, padd(d, e)); jz = padd(jz, psub(d, e));
-    dr = padd(faces, padd(padd(xy, xz), yz));
-    pxx = padd(s1, padd(xy, xz)); pyy = padd(s3, padd(xy, yz)); pzz = padd(s5, padd(xz, yz));
+  if constexpr (REF) {
+    const f2 lo = padd(padd(IO::to_f2(w[0]), sum(1)), padd(sum(3), sum(5)));
+    const f2 mid = padd(padd(sum(7), sum(9)), padd(sum(11), sum(13))), hi = padd(sum(15), sum(17));
+    dr = AR == ARITH_DIRECT ? padd(padd(lo, mid), hi) : padd(lo, padd(mid, hi));
+    jx = padd(padd(padd(dif(1), dif(7)), padd(dif(9), dif(11))), dif(13));
+    jy = padd(psub(padd(dif(3), dif(7)), dif(9)), padd(dif(15), dif(17)));
+    jz = padd(psub(padd(dif(5), dif(11)), dif(13)), psub(dif(15), dif(17)));
   } else {
     const f2 f0 = IO::to_f2(w[0]);
     f2 fa = IO::to_f2(w[1]), fb = IO::to_f2(w[2]);
@@ -489,19 +499,106 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
   }
   // ---- macroscopic state, relaxation rates -------------------------------
   const f2 r = padd(pk(SC), dr);
-  const f2 inv = prcp(r);
+  const f2 inv = AR == ARITH_DIRECT ? prcp_rn(r) : prcp(r);
   const f2 vx = pmul(jx, inv), vy = pmul(jy, inv), vz = pmul(jz, inv);
-  const f2 mx = MOM ? jx : vx, my = MOM ? jy : vy, mz = MOM ? jz : vz;
-  const f2 usq = pfma(mz, mz, pfma(my, my, pmul(mx, mx)));
-  const f2 A = pfma(pmul(pk(-1.5f), MOM ? inv : r), usq, dr);   // dr - 1.5 r u^2 (raw)
+  const f2 usq = REF && AR != ARITH_LEAN ? pfma(vz, vz, psq2(vx, vy))
+                                         : pfma(vz, vz, pfma(vy, vy, pmul(vx, vx)));
+  const f2 A = pfma(pmul(pk(-1.5f), r), usq, dr);   // dr - 1.5 r u^2 (raw)
   const bool ok0 = !fluid0 || (r.x > 0.0f && r.x < 3.0e38f);
   const bool ok1 = !fluid1 || (r.y > 0.0f && r.y < 3.0e38f);
   if (!(ok0 && ok1)) atomicOr(a.err, 1u);
   f2 om = pk(a.omega0f), omm = pk(a.omm0f);
-  if (a.les) {
+  // REF: the one-cell kernels' update. Per opposite pair (a, b), c = c_a . u:
+  //   sp = s/2 - w (A + 4.5 r c^2), sm = d/2 - 3 w r c   (weights negated below)
+  //   g_a = f_a - om sp - omm sm, g_b = f_b - om sp + omm sm
+  // sp is formed twice, for the stress and for the outputs, as its nine pairs
+  // do not fit in registers.
+  constexpr float WF = (float)(1.0 / 18), WE = (float)(1.0 / 36), W0 = (float)(1.0 / 3);
+  const f2 r3 = pmul(pk(3.0f), r), r45 = pmul(pk(4.5f), r);
+  const f2 nwAF = pmul(pk(-WF), A), nwAE = pmul(pk(-WE), A);
+  const f2 nw45F = AR == ARITH_LEAN ? pmul(pk(-4.5f * WF), r) : pmul(pk(-WF), r45);
+  const f2 nw45E = AR == ARITH_LEAN ? pmul(pk(-4.5f * WE), r) : pmul(pk(-WE), r45);
+  const f2 nw3F = AR == ARITH_LEAN ? pmul(pk(-3.0f * WF), r) : pmul(pk(-WF), r3);
+  const f2 nw3E = AR == ARITH_LEAN ? pmul(pk(-3.0f * WE), r) : pmul(pk(-WE), r3);
+  auto part_s = [&](int q, f2 c, f2 s) {   // sp of pair (q, q+1)
+    if constexpr (AR == ARITH_PBB) {
+      const f2 t = pfma(pmul(r45, c), c, A);
+      return pfma(pk(0.5f), s, pmul(pk(q < 7 ? -WF : -WE), t));
+    } else {
+      return pfma(pk(0.5f), s, pfma(pmul(q < 7 ? nw45F : nw45E, c), c, q < 7 ? nwAF : nwAE));
+    }
+  };
+  // keeps the compiler from carrying a pass's sums, differences and sp to the
+  // next pass in registers
+  auto forget = [&]() {
+#pragma unroll
+    for (int q = 0; q < Q; q++) IO::opaque(w[q]);
+  };
+  auto then = [&](int q, f2& after) {
+    asm volatile("" : "+f"(after.x), "+f"(after.y));
+    IO::opaque(w[q]);
+    IO::opaque(w[q + 1]);
+  };
+  if constexpr (REF) {
+    forget();
+    if (a.les) {
+      // two or three pairs at a time: `then` ties the next ones' words to the
+      // last sums, or all nine conversions run ahead and spill
+      f2 p7 = part_s(7, padd(vx, vy), sum(7)), p9 = part_s(9, psub(vx, vy), sum(9));
+      f2 sxy = psub(p7, p9);
+      then(11, sxy);
+      then(13, sxy);
+      f2 p11 = part_s(11, padd(vx, vz), sum(11)), p13 = part_s(13, psub(vx, vz), sum(13));
+      f2 sxz = psub(p11, p13), b = padd(p9, p11);
+      then(15, b);
+      then(17, b);
+      f2 p15 = part_s(15, padd(vy, vz), sum(15)), p17 = part_s(17, psub(vy, vz), sum(17));
+      f2 syz = psub(p15, p17), c = padd(p9, p15), e = padd(p13, p15);
+      then(1, e);
+      then(3, e);
+      then(5, e);
+      f2 sxx = padd(padd(padd(part_s(1, vx, sum(1)), p7), b), p13);
+      f2 syy = padd(padd(padd(part_s(3, vy, sum(3)), p7), c), p17);
+      f2 szz = padd(padd(padd(part_s(5, vz, sum(5)), p11), e), p17);
+      if constexpr (AR == ARITH_LEAN) {
+        const f2 off = pfma(syz, syz, pfma(sxz, sxz, pmul(sxy, sxy)));
+        const f2 q2 = pfma(sxx, sxx, pfma(syy, syy, pfma(szz, szz, padd(off, off))));
+        const f2 x = pmul(pmul(pk(a.les_cf), psqrt(q2)), inv);
+        const f2 te =
+            pfma(pk(0.5f), psqrt(pfma(pk(a.tau0f), pk(a.tau0f), x)), pk(0.5f * a.tau0f));
+        om = prcp(te);
+        const f2 t5 = psub(te, pk(0.5f));
+        omm = a.trt ? pmul(t5, prcp(pfma(pk(0.5f), t5, pk(a.lamf)))) : om;
+      } else {
+        if constexpr (AR == ARITH_PBB) {
+          sxx = padd(sxx, sxx); syy = padd(syy, syy); szz = padd(szz, szz);
+          sxy = padd(sxy, sxy); sxz = padd(sxz, sxz); syz = padd(syz, syz);
+        }
+        const f2 off = pfma(syz, syz, psq2(sxy, sxz));
+        const f2 q2 = pfma(pk(2.0f), off, pfma(szz, szz, psq2(sxx, syy)));
+        if constexpr (AR == ARITH_DIRECT) {
+          const f2 x = pmul(pmul(pk(a.les_cf), psqrt_rn(q2)), inv);
+          const f2 te = pmul(
+              pk(0.5f), padd(pk(a.tau0f), psqrt_rn(pfma(pk(a.tau0f), pk(a.tau0f), x))));
+          om = prcp_rn(te);
+          const f2 t5 = psub(te, pk(0.5f)), t6 = pfma(pk(0.5f), t5, pk(a.lamf));
+          omm = a.trt ? make_float2(__fdividef(t5.x, t6.x), __fdividef(t5.y, t6.y)) : om;
+        } else {
+          const float k = (float)(18 * 1.4142135623730951) * (float)a.cs2;
+          const f2 x = pmul(pmul(pk(k), psqrt(padd(q2, q2))), inv);
+          const f2 te =
+              pmul(pk(0.5f), padd(pk(a.tau0f), psqrt(pfma(pk(a.tau0f), pk(a.tau0f), x))));
+          om = prcp(te);
+          omm = a.trt ? prcp(pfma(pk(a.lamf), prcp(psub(te, pk(0.5f))), pk(0.5f))) : om;
+        }
+      }
+    } else if constexpr (AR == ARITH_PBB) {
+      om = prcp(pk(a.tau0f));
+      omm = a.trt ? prcp(pfma(pk(a.lamf), prcp(psub(pk(a.tau0f), pk(0.5f))), pk(0.5f))) : om;
+    }
+  } else if (a.les) {
     // non-equilibrium second moments: P - (dr/3 + r u u), js/lbm.js:420-425
-    const f2 rvx = MOM ? jx : pmul(r, vx), rvy = MOM ? jy : pmul(r, vy),
-             rvz = MOM ? jz : pmul(r, vz);
+    const f2 rvx = pmul(r, vx), rvy = pmul(r, vy), rvz = pmul(r, vz);
     const f2 dr3 = pmul(pk(1.0f / 3.0f), dr);
     const f2 sxx = pfma(pmul(pk(-1.0f), rvx), vx, psub(pxx, dr3));
     const f2 syy = pfma(pmul(pk(-1.0f), rvy), vy, psub(pyy, dr3));
@@ -513,11 +610,8 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     const f2 q2 = pfma(sxx, sxx, pfma(syy, syy, pfma(szz, szz, padd(off, off))));
     // 18 sqrt(2) Cs^2 |Pi| / rho with |Pi| = sqrt(2 q2): 36 Cs^2 sqrt(q2) / r
     const f2 x = pmul(pmul(pk(0.5f * a.les_cf), psqrt(q2)), inv);
-    const f2 rad = pfma(pk(a.tau0f), pk(a.tau0f), x);
-    // MOV stands for the direct kernel, whose square root and reciprocal round
-    const f2 root = MOV ? make_float2(__fsqrt_rn(rad.x), __fsqrt_rn(rad.y)) : psqrt(rad);
-    const f2 te = pfma(pk(0.5f), root, pk(0.5f * a.tau0f));
-    om = MOV ? make_float2(__frcp_rn(te.x), __frcp_rn(te.y)) : prcp(te);
+    const f2 te = pfma(pk(0.5f), psqrt(pfma(pk(a.tau0f), pk(a.tau0f), x)), pk(0.5f * a.tau0f));
+    om = prcp(te);
     if (a.trt) {
       const f2 t5 = psub(te, pk(0.5f));
       omm = pmul(t5, prcp(pfma(pk(0.5f), t5, pk(a.lamf))));
@@ -568,39 +662,30 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
   // (s = f_a + f_b, d = f_a - f_b, c = c_a . u); w = 1/18 face, 1/36 edge
   const f2 al = pfma(pk(-0.5f), om, pk(0.5f));
   const f2 be = pfma(pk(-0.5f), omm, pk(0.5f));
-  // MOM: g_a = f_a + (om T + omm U), g_b = f_b + (om T - omm U) with
-  //   T = w (A + 4.5 c^2 / r) - s/2,  U = 3 w c - d/2  (c = c_a . j),
-  // A/36 and j/12 formed with the constants' remainders and the faces and the
-  // rest cell taken as 2 and 12 times the edges' value, so that the sums of the
-  // weights are not off by the constants' rounding (3e-8 of the momentum a step)
-  auto over = [](f2 v, double d) {
-    const float hi = (float)(1.0 / d), lo = (float)(1.0 / d - (double)(float)(1.0 / d));
-    return pfma(v, pk(hi), pmul(v, pk(lo)));
-  };
   const f2 omr = pmul(om, r), ommr = pmul(omm, r), omA = pmul(om, A);
-  const f2 kae = MOM ? over(A, 36.0) : pmul(pk((float)(1.0 / 36)), omA);
-  const f2 kaf = MOM ? padd(kae, kae) : pmul(pk((float)(1.0 / 18)), omA);
-  const f2 k45f = pmul(pk(0.25f), MOM ? inv : omr), k45e = pmul(pk(0.125f), MOM ? inv : omr);
+  const f2 k45f = pmul(pk(0.25f), omr), k45e = pmul(pk(0.125f), omr);
+  const f2 kaf = pmul(pk((float)(1.0 / 18)), omA), kae = pmul(pk((float)(1.0 / 36)), omA);
   const f2 k3f = pmul(pk((float)(1.0 / 6)), ommr), k3e = pmul(pk((float)(1.0 / 12)), ommr);
-  const f2 hx = over(jx, 12.0), hy = over(jy, 12.0), hz = over(jz, 12.0);   // MOM only
   // a solid cell keeps its stale populations, and so does the outlet copy
   // of a solid cell nx-2 until the copy below
   const bool keep0 = solid0 && !inlet, keep1 = solid1 || (outlet && solid0);
   const bool keep_any = keep0 || keep1;
   // stochastic rounding: a hash of (pair, step), then per output word its
-  // product with a distinct odd constant (one multiply per word)
-  uint32_t h = 0;
-  if constexpr (SR) {
-    h = ((uint32_t)i0 ^ (uint32_t)(i0 >> 32)) * 0x9E3779B1u ^ a.sr_seed;
-    h ^= h >> 16; h *= 0x85EBCA6Bu; h ^= h >> 13; h *= 0xC2B2AE35u; h ^= h >> 16;
-  }
-  auto put = [&](int q, f2 g) {
-    W v;
-    if constexpr (SR) {
-      v = IO::pack_sr(g, h * (0x9E3779B1u * (2u * (uint32_t)q + 1u)));
-    } else {
-      v = IO::pack(g);
-    }
+  // product with a distinct odd constant (one multiply per word); REF: the
+  // one-cell kernels' chain of each of the two cells, 32 bits per opposite pair
+  auto mix = [&](long long i) {
+    uint32_t v = ((uint32_t)i ^ (uint32_t)(i >> 32)) * 0x9E3779B1u ^ a.sr_seed;
+    v ^= v >> 16; v *= 0x85EBCA6Bu; v ^= v >> 13; v *= 0xC2B2AE35u; v ^= v >> 16;
+    return v;
+  };
+  auto next = [](uint32_t v) {
+    v ^= v << 13; v ^= v >> 17; v ^= v << 5;
+    return v;
+  };
+  uint32_t h = 0, h1 = 0;
+  if constexpr (SR) h = mix(i0);
+  if constexpr (SR && REF) h1 = mix(i0 + 1);
+  auto store = [&](int q, W v) {
     // the inlet's low cell takes the equilibrium, the outlet's high cell
     // takes cell nx-2's value
     v = IO::fix(v, IO::eq(a, q), inlet, outlet);
@@ -616,59 +701,82 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
       if (!keep1) gh(q, 1) = IO::lane(v, 1);
     }
   };
+  auto put = [&](int q, f2 g) {
+    if constexpr (SR) store(q, IO::pack_sr(g, h * (0x9E3779B1u * (2u * (uint32_t)q + 1u))));
+    else store(q, IO::pack(g));
+  };
+  auto put2 = [&](int q, f2 ga, f2 gb) {   // the pair (q, q+1)
+    if constexpr (SR && REF) {
+      h = next(h);
+      h1 = next(h1);
+      const W x = IO::pack_sr(make_float2(gb.x, ga.x), h), y = IO::pack_sr(make_float2(gb.y, ga.y), h1);
+      store(q, IO::highs(x, y));
+      store(q + 1, IO::lows(x, y));
+    } else {
+      put(q, ga);
+      put(q + 1, gb);
+    }
+  };
   // ---- pass 2: outputs ----------------------------------------------------
   const f2 s1 = psub(pk(1.0f), sf);   // BLEND only
-  {
+  if constexpr (REF) {
+    forget();
+    const f2 nom = pmul(pk(-1.0f), om), nomm = pmul(pk(-1.0f), omm);
+    auto out = [&](int q, f2 c) {
+      const f2 fa = IO::to_f2(w[q]), fb = IO::to_f2(w[q + 1]);
+      const f2 s = padd(fa, fb), d = psub(fa, fb);
+      const f2 sp = part_s(q, c, s), sm = pfma(pk(0.5f), d, pmul(q < 7 ? nw3F : nw3E, c));
+      f2 ga = pfma(nomm, sm, pfma(nom, sp, fa)), gb = pfma(omm, sm, pfma(nom, sp, fb));
+      if constexpr (BLEND) {
+        // c_a (g_a - f_b) + c_b (g_b - f_a), c_b = -c_a
+        const f2 e = padd(psub(ga, gb), d);
+        if (ex(q) == 1) F[0] = padd(F[0], e);
+        if (ey(q) == 1) F[1] = padd(F[1], e);
+        if (ez(q) == 1) F[2] = padd(F[2], e);
+        if (ey(q) == -1) F[1] = psub(F[1], e);
+        if (ez(q) == -1) F[2] = psub(F[2], e);
+        ga = pfma(sf, fb, pmul(s1, ga));
+        gb = pfma(sf, fa, pmul(s1, gb));
+      }
+      put2(q, ga, gb);
+    };
+    out(1, vx); out(3, vy); out(5, vz);
+    out(7, padd(vx, vy)); out(9, psub(vx, vy)); out(11, padd(vx, vz));
+    out(13, psub(vx, vz)); out(15, padd(vy, vz)); out(17, psub(vy, vz));
     const f2 f0 = IO::to_f2(w[0]);
-    if constexpr (MOM) {
-      f2 g = pfma(om, pfma(pk(12.0f), kae, pmul(pk(-1.0f), f0)), f0);
-      if constexpr (BLEND) g = pfma(sf, f0, pmul(s1, g));
-      put(0, g);
+    f2 g0 = pfma(nom, pfma(pk(-W0), A, f0), f0);
+    if constexpr (BLEND) g0 = pfma(sf, f0, pmul(s1, g0));
+    if constexpr (SR) {
+      h = next(h);
+      h1 = next(h1);
+      store(0, IO::lows(IO::pack_sr(make_float2(g0.x, 0.0f), h), IO::pack_sr(make_float2(g0.y, 0.0f), h1)));
+    } else {
+      store(0, IO::pack(g0));
     }
-    else
-      put(0, pfma(pfma(pk(-1.0f), om, pk(1.0f)), f0, pmul(pk((float)(1.0 / 3)), omA)));
-  }
-#define WT_PAIR_OUT(qa, C, H, K45, KA, K3)                          \
+  } else {
+    const f2 f0 = IO::to_f2(w[0]);
+    put(0, pfma(pfma(pk(-1.0f), om, pk(1.0f)), f0, pmul(pk((float)(1.0 / 3)), omA)));
+#define WT_PAIR_OUT(qa, C, K45, KA, K3)                             \
   {                                                                 \
     const f2 fa = IO::to_f2(w[qa]), fb = IO::to_f2(w[qa + 1]);      \
     const f2 s = padd(fa, fb), d = psub(fa, fb);                    \
     const f2 c = C;                                                 \
     const f2 X = pfma(pmul(c, c), K45, KA);                         \
-    if constexpr (MOM) {                                            \
-      const f2 T = pmul(om, pfma(pk(-0.5f), s, X));                 \
-      const f2 U = pfma(pk(-0.5f), d, H);                           \
-      f2 ga = padd(fa, pfma(omm, U, T));                            \
-      f2 gb = padd(fb, pfma(pmul(pk(-1.0f), omm), U, T));           \
-      if constexpr (BLEND) {                                        \
-        /* c_a (g_a - f_b) + c_b (g_b - f_a), c_b = -c_a */         \
-        const f2 e = padd(psub(ga, gb), d);                         \
-        if constexpr (ex(qa) == 1) F[0] = padd(F[0], e);            \
-        if constexpr (ey(qa) == 1) F[1] = padd(F[1], e);            \
-        if constexpr (ez(qa) == 1) F[2] = padd(F[2], e);            \
-        if constexpr (ey(qa) == -1) F[1] = psub(F[1], e);           \
-        if constexpr (ez(qa) == -1) F[2] = psub(F[2], e);           \
-        ga = pfma(sf, fb, pmul(s1, ga));                            \
-        gb = pfma(sf, fa, pmul(s1, gb));                            \
-      }                                                             \
-      put(qa, ga);                                                  \
-      put(qa + 1, gb);                                              \
-    } else {                                                        \
-      const f2 Y = pmul(K3, c);                                     \
-      const f2 P = pfma(al, s, X), M = pfma(be, d, Y);              \
-      put(qa, padd(P, M));                                          \
-      put(qa + 1, psub(P, M));                                      \
-    }                                                               \
+    const f2 Y = pmul(K3, c);                                       \
+    const f2 P = pfma(al, s, X), M = pfma(be, d, Y);                \
+    put2(qa, padd(P, M), psub(P, M));                               \
   }
-  WT_PAIR_OUT(1, mx, padd(hx, hx), k45f, kaf, k3f)
-  WT_PAIR_OUT(3, my, padd(hy, hy), k45f, kaf, k3f)
-  WT_PAIR_OUT(5, mz, padd(hz, hz), k45f, kaf, k3f)
-  WT_PAIR_OUT(7, padd(mx, my), padd(hx, hy), k45e, kae, k3e)
-  WT_PAIR_OUT(9, psub(mx, my), psub(hx, hy), k45e, kae, k3e)
-  WT_PAIR_OUT(11, padd(mx, mz), padd(hx, hz), k45e, kae, k3e)
-  WT_PAIR_OUT(13, psub(mx, mz), psub(hx, hz), k45e, kae, k3e)
-  WT_PAIR_OUT(15, padd(my, mz), padd(hy, hz), k45e, kae, k3e)
-  WT_PAIR_OUT(17, psub(my, mz), psub(hy, hz), k45e, kae, k3e)
+    WT_PAIR_OUT(1, vx, k45f, kaf, k3f)
+    WT_PAIR_OUT(3, vy, k45f, kaf, k3f)
+    WT_PAIR_OUT(5, vz, k45f, kaf, k3f)
+    WT_PAIR_OUT(7, padd(vx, vy), k45e, kae, k3e)
+    WT_PAIR_OUT(9, psub(vx, vy), k45e, kae, k3e)
+    WT_PAIR_OUT(11, padd(vx, vz), k45e, kae, k3e)
+    WT_PAIR_OUT(13, psub(vx, vz), k45e, kae, k3e)
+    WT_PAIR_OUT(15, padd(vy, vz), k45e, kae, k3e)
+    WT_PAIR_OUT(17, psub(vy, vz), k45e, kae, k3e)
 #undef WT_PAIR_OUT
+  }
   if (outlet && solid0) {
     // copy of a solid cell nx-2, whose g this step does not write
     R v[Q];
@@ -747,7 +855,7 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
     else fl = ld16(reinterpret_cast<const char*>(a.flags + i0));
   }
   W w[Q];
-#define WT_PAIR_JOIN(q) w[q] = IO::template join<ex(q)>(raw[q]);
+#define WT_PAIR_JOIN(q) w[q] = IO::template join<ex(q), ODD>(raw[q]);
   WT_EACH_Q(WT_PAIR_JOIN)
 #undef WT_PAIR_JOIN
   const PairCells c = pair_cells<MODE>(fl, x0, a.nx);

@@ -36,6 +36,12 @@ __device__ __forceinline__ f2 psub(f2 a, f2 b) {
 __device__ __forceinline__ f2 prcp(f2 a) { return make_float2(rcp_approx(a.x), rcp_approx(a.y)); }
 __device__ __forceinline__ f2 psqrt(f2 a) { return make_float2(sqrt_approx(a.x), sqrt_approx(a.y)); }
 
+// Correctly rounded forms (the direct kernel's in float32), and x^2 + y^2 as the
+// compiler contracts it: the first product in the fused operation.
+__device__ __forceinline__ f2 prcp_rn(f2 a) { return make_float2(__frcp_rn(a.x), __frcp_rn(a.y)); }
+__device__ __forceinline__ f2 psqrt_rn(f2 a) { return make_float2(__fsqrt_rn(a.x), __fsqrt_rn(a.y)); }
+__device__ __forceinline__ f2 psq2(f2 x, f2 y) { return pfma(x, x, pmul(y, y)); }
+
 // The same operations on one cell (a scalar float), so that the collision
 // below also serves the one-cell-per-thread kernels.
 template <class V>
