@@ -74,9 +74,7 @@ long long range_cells(const int rg[6]) {
 }
 
 void free_all(wt_lattice* h) {
-  void* dev[] = {h->buf[0], h->buf[1], h->flags, h->nmask, h->ux, h->uy, h->uz, h->rho, h->uwx, h->uwy,
-                 h->uwz, h->part, h->wslot, h->segmark, h->slot_scan, h->sfrac_buf, h->err_dev,
-                 h->vstats, h->vox_in};
+  void* dev[] = {h->block, h->part, h->sfrac_buf, h->vox_in};
   for (void* p : dev)
     if (p) cudaFree(p);
   if (h->forces_host) cudaFreeHost(h->forces_host);
@@ -411,23 +409,38 @@ int wt_create(int nx, int ny, int nz, int storage, wt_lattice** out) {
     return WT_ERR_CUDA;
   }
   bool ok = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->buf[0], pop) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->buf[1], pop) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->flags, (size_t)n) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->nmask, sizeof(unsigned long long) * (size_t)n) == cudaSuccess;
-  float** fl[] = {&h->ux, &h->uy, &h->uz, &h->rho, &h->uwx, &h->uwy, &h->uwz};
-  for (float** p : fl) ok = ok && cudaMalloc((void**)p, sizeof(float) * (size_t)n) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->wslot, sizeof(int) * (size_t)h->nsegs) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->err_dev, sizeof(unsigned)) == cudaSuccess;
-  ok = ok && cudaMallocHost((void**)&h->err_host, sizeof(unsigned)) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->segmark, (size_t)h->nsegs) == cudaSuccess;
-  ok = ok && cudaMalloc((void**)&h->slot_scan, sizeof(int) * wt::slot_scan_ints(h)) == cudaSuccess;
+  // one block for everything of the lattice's size: a cudaMalloc is up to a
+  // millisecond, and there were nineteen
   h->vstats_bytes = 8 + 5 * (size_t)nx * nz + (size_t)ny * nz;
-  ok = ok && cudaMalloc((void**)&h->vstats, h->vstats_bytes) == cudaSuccess;
-  h->counters = (int*)h->vstats;
-  h->low = h->counters + 2;
-  h->col = (uint8_t*)(h->low + (size_t)nx * nz);
-  h->plan = h->col + (size_t)ny * nz;
+  const size_t cells = (size_t)n;
+  struct Part {
+    void** p;
+    size_t bytes;
+  } parts[] = {{&h->buf[0], pop}, {&h->buf[1], pop}, {(void**)&h->flags, cells},
+               {(void**)&h->nmask, sizeof(unsigned long long) * cells},
+               {(void**)&h->ux, sizeof(float) * cells}, {(void**)&h->uy, sizeof(float) * cells},
+               {(void**)&h->uz, sizeof(float) * cells}, {(void**)&h->rho, sizeof(float) * cells},
+               {(void**)&h->uwx, sizeof(float) * cells}, {(void**)&h->uwy, sizeof(float) * cells},
+               {(void**)&h->uwz, sizeof(float) * cells},
+               {(void**)&h->wslot, sizeof(int) * (size_t)h->nsegs},
+               {(void**)&h->segmark, (size_t)h->nsegs},
+               {(void**)&h->slot_scan, sizeof(int) * (size_t)wt::slot_scan_ints(h)},
+               {(void**)&h->vstats, h->vstats_bytes}, {(void**)&h->err_dev, sizeof(unsigned)}};
+  size_t total = 0;
+  for (const Part& q : parts) total += (q.bytes + 511) & ~(size_t)511;
+  ok = ok && cudaMalloc(&h->block, total) == cudaSuccess;
+  if (ok) {
+    unsigned char* at = (unsigned char*)h->block;
+    for (const Part& q : parts) {
+      *q.p = at;
+      at += (q.bytes + 511) & ~(size_t)511;
+    }
+    h->counters = (int*)h->vstats;
+    h->low = h->counters + 2;
+    h->col = (uint8_t*)(h->low + (size_t)nx * nz);
+    h->plan = h->col + (size_t)ny * nz;
+  }
+  ok = ok && cudaMallocHost((void**)&h->err_host, sizeof(unsigned)) == cudaSuccess;
   ok = ok && grow_forces(h, 64) == WT_OK;
   if (!ok) {
     cudaGetLastError();

@@ -20,6 +20,7 @@ struct wt_lattice {
   size_t elem = 4;               // bytes per stored population
   cudaStream_t stream = nullptr;
   cudaStream_t aux = nullptr;    // second stream of wt_adjoint (recomputation), made on first use
+  void* block = nullptr;         // the device memory of the pointers down to err_dev
   void* buf[2] = {nullptr, nullptr};  // population buffers A and B (js/lbm.js:74-75)
   int parity = 0;                // js/lbm.js:80: f = parity ? B : A
   uint8_t* flags = nullptr;      // solid code (bits 0-1) | near bit (bit 2)
