@@ -178,85 +178,10 @@ __device__ __forceinline__ void cell_fw(const StepArgs<S>& a, CellFw<T>& c) {
   c.usq = usq; c.A = A; c.r3 = r3; c.r45 = r45; c.tauEff = tauEff; c.om = om; c.omm = omm;
 }
 
-// The float32 form of cell_vjp, over the nine opposite pairs: with
-// P = nb_a + nb_b and D = nb_a - nb_b (the adjoints of the pair's
-// symmetric and antisymmetric non-equilibrium parts), the stress terms add
-// to P only, and the equilibrium's adjoint needs each pair once (c_b = -c_a).
-template <class S>
-__device__ __forceinline__ void cell_vjp_pairs(const StepArgs<S>& a, const CellFw<float>& c,
-                                               const float (&ab)[Q], float (&fb)[Q]) {
-  const float* n = c.n;
-  float P[Q], D[Q];   // indexed by the pair's first direction (1, 3, ..., 17)
-  float omb = -(ab[0] * n[0]);
-  float ommb = 0.0f;
-  const float nb0 = -(c.om * ab[0]);
-#pragma unroll
-  for (int k = 1; k < Q; k += 2) {
-    const float sp = 0.5f * (n[k] + n[k + 1]), sm = 0.5f * (n[k] - n[k + 1]);
-    const float as = ab[k] + ab[k + 1], ad = ab[k] - ab[k + 1];
-    omb -= as * sp;
-    ommb -= ad * sm;
-    P[k] = -(c.om * as);
-    D[k] = -(c.omm * ad);
-  }
-  float invb = 0.0f;
-  if (a.les) {
-    float teb;
-    if (a.trt) {
-      const float tm = c.tauEff - 0.5f;
-      teb = ommb * cdiv(c.omm * c.omm * (float)a.lam, tm * tm) - omb * (c.om * c.om);
-    } else {
-      teb = -(omb + ommb) * (c.om * c.om);
-    }
-    const float Rb = 0.5f * teb;
-    const float Xb = cdiv(Rb, 2.0f * c.R);
-    const float K = (float)(18 * 1.4142135623730951) * (float)a.cs2;
-    const float magb = Xb * K * c.inv;
-    invb += Xb * K * c.mag;
-    const float Qb = c.mag > 0.0f ? cdiv(magb, c.mag) : 0.0f;
-    const float pxxb = 4.0f * c.pxx * Qb, pyyb = 4.0f * c.pyy * Qb, pzzb = 4.0f * c.pzz * Qb;
-    const float pxyb = 8.0f * c.pxy * Qb, pxzb = 8.0f * c.pxz * Qb, pyzb = 8.0f * c.pyz * Qb;
-    P[1] += pxxb; P[3] += pyyb; P[5] += pzzb;
-    P[7] += pxxb + pyyb + pxyb; P[9] += pxxb + pyyb - pxyb;
-    P[11] += pxxb + pzzb + pxzb; P[13] += pxxb + pzzb - pxzb;
-    P[15] += pyyb + pzzb + pyzb; P[17] += pyyb + pzzb - pyzb;
-  }
-  float Ab = (float)wq(0) * (-nb0), r3b = 0.0f, r45b = 0.0f, vxb = 0.0f, vyb = 0.0f, vzb = 0.0f;
-#pragma unroll
-  for (int k = 1; k < Q; k += 2) {
-    const float E = -P[k], Dm = -D[k], w = (float)wq(k);
-    const float cv = (float)ex(k) * c.vx + (float)ey(k) * c.vy + (float)ez(k) * c.vz;
-    Ab += w * E;
-    r3b += w * cv * Dm;
-    r45b += w * (cv * cv) * E;
-    const float cvbd = w * (c.r3 * Dm + 2.0f * c.r45 * cv * E);
-    vxb += (float)ex(k) * cvbd; vyb += (float)ey(k) * cvbd; vzb += (float)ez(k) * cvbd;
-  }
-  float drb = Ab;
-  float rb = 3.0f * r3b + 4.5f * r45b - 1.5f * c.usq * Ab;
-  const float usqb = -(c.r * 1.5f * Ab);
-  vxb += 2.0f * c.vx * usqb; vyb += 2.0f * c.vy * usqb; vzb += 2.0f * c.vz * usqb;
-  invb += vxb * c.jx + vyb * c.jy + vzb * c.jz;
-  const float jxb = vxb * c.inv, jyb = vyb * c.inv, jzb = vzb * c.inv;
-  rb -= c.inv * c.inv * invb;
-  drb += rb;
-  fb[0] += ab[0] + nb0 + drb;
-#pragma unroll
-  for (int k = 1; k < Q; k += 2) {
-    const float cj = (float)ex(k) * jxb + (float)ey(k) * jyb + (float)ez(k) * jzb;
-    fb[k] += ab[k] + 0.5f * (P[k] + D[k]) + (drb + cj);
-    fb[k + 1] += ab[k + 1] + 0.5f * (P[k] - D[k]) + (drb - cj);
-  }
-}
-
 // fb += (d gc / d f)^T a for the collision of cell_fw.
 template <class T, class S>
 __device__ __forceinline__ void cell_vjp(const StepArgs<S>& a, const CellFw<T>& c, const T (&ab)[Q],
                                          T (&fb)[Q]) {
-  if constexpr (std::is_same<T, float>::value) {
-    cell_vjp_pairs(a, c, ab, fb);
-    return;
-  }
   const T* n = c.n;
   T nb[Q];
 #pragma unroll
@@ -492,6 +417,191 @@ __device__ __forceinline__ T adj_shell(const StepArgs<S>& a, const T* Tn, int q,
   return v;
 }
 
+// The float32 adjoint of one cell's collision, over its nine opposite pairs
+// (a, b). With s = f_a + f_b, d = f_a - f_b and c = c_a . u the pair's symmetric
+// and antisymmetric non-equilibrium parts are
+//   sp = s/2 - w (A + 4.5 r c^2),   sm = d/2 - 3 w r c;
+// P and D, their adjoints, start as -om (g_a + g_b) and -omm (g_a - g_b), the stress
+// adds to P, and the equilibrium's adjoint needs each pair once (c_b = -c_a).
+// Two pairs are computed at a time in packed float32x2 instructions within the
+// cell: (7,9), (11,13), (15,17), (1,3) in two lanes, 5 alone, which halves the
+// floating-point instructions without the two cells' registers that a pair of
+// cells per thread needs.
+struct AdjPairs {
+  float2 e1, e2, e3, f1;   // pairs (7,9), (11,13), (15,17) and (1,3)
+  float f5;                // pair 5
+};
+__device__ __forceinline__ float2 p2(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ float2 p2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 a2(float2 x, float2 y) { return __fadd2_rn(x, y); }
+__device__ __forceinline__ float2 m2(float2 x, float2 y) { return __fmul2_rn(x, y); }
+__device__ __forceinline__ float2 fm2(float2 x, float2 y, float2 z) { return __ffma2_rn(x, y, z); }
+__device__ __forceinline__ float2 s2(float2 x, float2 y) { return __ffma2_rn(p2(-1.0f), y, x); }
+__device__ __forceinline__ float fm2(float x, float y, float z) { return fmaf(x, y, z); }
+
+// State of the forward collision that the adjoint needs.
+struct AdjCell {
+  AdjPairs sp, sm;
+  float n0, r, inv, jx, jy, jz, vx, vy, vz, usq, om, omm, tauEff, mag, R;
+  float pxx, pyy, pzz, pxy, pxz, pyz;
+};
+
+// The values of first directions (7, 9, ...) and of second ones (8, 10, ...).
+__device__ __forceinline__ AdjPairs firsts(const float (&v)[Q]) {
+  return AdjPairs{p2(v[7], v[9]), p2(v[11], v[13]), p2(v[15], v[17]), p2(v[1], v[3]), v[5]};
+}
+__device__ __forceinline__ AdjPairs seconds(const float (&v)[Q]) {
+  return AdjPairs{p2(v[8], v[10]), p2(v[12], v[14]), p2(v[16], v[18]), p2(v[2], v[4]), v[6]};
+}
+__device__ __forceinline__ AdjPairs operator+(const AdjPairs& x, const AdjPairs& y) {
+  return AdjPairs{a2(x.e1, y.e1), a2(x.e2, y.e2), a2(x.e3, y.e3), a2(x.f1, y.f1), x.f5 + y.f5};
+}
+__device__ __forceinline__ AdjPairs operator-(const AdjPairs& x, const AdjPairs& y) {
+  return AdjPairs{s2(x.e1, y.e1), s2(x.e2, y.e2), s2(x.e3, y.e3), s2(x.f1, y.f1), x.f5 - y.f5};
+}
+// c_a . v of every pair
+__device__ __forceinline__ AdjPairs along(float x, float y, float z) {
+  return AdjPairs{p2(x + y, x - y), p2(x + z, x - z), p2(y + z, y - z), p2(x, y), z};
+}
+// sum over the pairs of c_a (a vector) times the pair's value
+__device__ __forceinline__ void moment(const AdjPairs& v, float& x, float& y, float& z) {
+  x = v.f1.x + ((v.e1.x + v.e1.y) + (v.e2.x + v.e2.y));
+  y = v.f1.y + ((v.e1.x - v.e1.y) + (v.e3.x + v.e3.y));
+  z = v.f5 + ((v.e2.x - v.e2.y) + (v.e3.x - v.e3.y));
+}
+
+template <class S>
+__device__ __forceinline__ void adj_forward(const StepArgs<S>& a, const float (&f)[Q], AdjCell& c) {
+  constexpr float WF = (float)(1.0 / 18), WE = (float)(1.0 / 36), W0 = (float)(1.0 / 3);
+  const AdjPairs fa = firsts(f), fb = seconds(f);
+  const AdjPairs s = fa + fb, d = fa - fb;
+  const float2 es = a2(a2(s.e1, s.e2), s.e3);
+  const float dr = (f[0] + (s.f1.x + s.f1.y)) + (s.f5 + (es.x + es.y));
+  c.r = 1.0f + dr;
+  c.inv = rcp_approx(c.r);
+  moment(d, c.jx, c.jy, c.jz);
+  c.vx = c.jx * c.inv; c.vy = c.jy * c.inv; c.vz = c.jz * c.inv;
+  c.usq = c.vx * c.vx + c.vy * c.vy + c.vz * c.vz;
+  const float A = dr - 1.5f * c.r * c.usq, r45 = 4.5f * c.r, r3 = 3.0f * c.r;
+  const AdjPairs cv = along(c.vx, c.vy, c.vz);
+  auto part2 = [&](float2 s_, float2 d_, float2 c_, float w, float2& sp, float2& sm) {
+    sp = fm2(p2(-w), fm2(m2(p2(r45), c_), c_, p2(A)), m2(p2(0.5f), s_));
+    sm = fm2(p2(-w * r3), c_, m2(p2(0.5f), d_));
+  };
+  part2(s.e1, d.e1, cv.e1, WE, c.sp.e1, c.sm.e1);
+  part2(s.e2, d.e2, cv.e2, WE, c.sp.e2, c.sm.e2);
+  part2(s.e3, d.e3, cv.e3, WE, c.sp.e3, c.sm.e3);
+  part2(s.f1, d.f1, cv.f1, WF, c.sp.f1, c.sm.f1);
+  c.sp.f5 = fmaf(-WF, fmaf(r45 * cv.f5, cv.f5, A), 0.5f * s.f5);
+  c.sm.f5 = fmaf(-WF * r3, cv.f5, 0.5f * d.f5);
+  c.n0 = fmaf(-W0, A, f[0]);
+  const float tau0 = a.tau0f;
+  c.tauEff = tau0;
+  c.om = rcp_approx(tau0);
+  c.pxx = c.pyy = c.pzz = c.pxy = c.pxz = c.pyz = c.mag = c.R = 0.0f;
+  if (a.les) {
+    const float xy = c.sp.e1.x + c.sp.e1.y, xz = c.sp.e2.x + c.sp.e2.y, yz = c.sp.e3.x + c.sp.e3.y;
+    c.pxx = 2.0f * (c.sp.f1.x + (xy + xz));
+    c.pyy = 2.0f * (c.sp.f1.y + (xy + yz));
+    c.pzz = 2.0f * (c.sp.f5 + (xz + yz));
+    c.pxy = 2.0f * (c.sp.e1.x - c.sp.e1.y);
+    c.pxz = 2.0f * (c.sp.e2.x - c.sp.e2.y);
+    c.pyz = 2.0f * (c.sp.e3.x - c.sp.e3.y);
+    c.mag = sqrt_approx(2.0f * (c.pxx * c.pxx + c.pyy * c.pyy + c.pzz * c.pzz +
+                                2.0f * (c.pxy * c.pxy + c.pxz * c.pxz + c.pyz * c.pyz)));
+    const float K = (float)(18 * 1.4142135623730951) * (float)a.cs2;
+    c.R = sqrt_approx(tau0 * tau0 + K * c.mag * c.inv);
+    c.tauEff = 0.5f * (tau0 + c.R);
+    c.om = rcp_approx(c.tauEff);
+  }
+  c.omm = a.trt ? rcp_approx(0.5f + a.lamf * rcp_approx(c.tauEff - 0.5f)) : c.om;
+}
+
+// out(q, v): v = the adjoint of the value pulled by link q, for adjoints ab of the
+// collided values.
+template <class S, class Out>
+__device__ __forceinline__ void adj_backward(const StepArgs<S>& a, const AdjCell& c,
+                                             const float (&ab)[Q], Out out) {
+  constexpr float WF = (float)(1.0 / 18), WE = (float)(1.0 / 36), W0 = (float)(1.0 / 3);
+  const AdjPairs ga = firsts(ab), gb = seconds(ab);
+  AdjPairs P = ga + gb, D = ga - gb;
+  float2 t = m2(P.e1, c.sp.e1);
+  t = fm2(P.e2, c.sp.e2, t); t = fm2(P.e3, c.sp.e3, t); t = fm2(P.f1, c.sp.f1, t);
+  const float omb = -(ab[0] * c.n0 + (P.f5 * c.sp.f5 + (t.x + t.y)));
+  t = m2(D.e1, c.sm.e1);
+  t = fm2(D.e2, c.sm.e2, t); t = fm2(D.e3, c.sm.e3, t); t = fm2(D.f1, c.sm.f1, t);
+  const float ommb = -(D.f5 * c.sm.f5 + (t.x + t.y));
+  // E and G: minus the adjoints P and D (the equilibrium enters with -1)
+  const float2 om2 = p2(c.om), omm2 = p2(c.omm);
+  AdjPairs E{m2(om2, P.e1), m2(om2, P.e2), m2(om2, P.e3), m2(om2, P.f1), c.om * P.f5};
+  const AdjPairs G{m2(omm2, D.e1), m2(omm2, D.e2), m2(omm2, D.e3), m2(omm2, D.f1), c.omm * D.f5};
+  const float e0 = c.om * ab[0];
+  float invb = 0.0f;
+  if (a.les) {
+    float teb;
+    if (a.trt) {
+      const float tm = c.tauEff - 0.5f;
+      teb = ommb * cdiv(c.omm * c.omm * a.lamf, tm * tm) - omb * (c.om * c.om);
+    } else {
+      teb = -(omb + ommb) * (c.om * c.om);
+    }
+    const float Xb = cdiv(0.5f * teb, 2.0f * c.R);
+    const float K = (float)(18 * 1.4142135623730951) * (float)a.cs2;
+    const float magb = Xb * K * c.inv;
+    invb = Xb * K * c.mag;
+    const float Qb = c.mag > 0.0f ? cdiv(magb, c.mag) : 0.0f;
+    const float xx = 4.0f * c.pxx * Qb, yy = 4.0f * c.pyy * Qb, zz = 4.0f * c.pzz * Qb;
+    const float xy = 8.0f * c.pxy * Qb, xz = 8.0f * c.pxz * Qb, yz = 8.0f * c.pyz * Qb;
+    E.e1 = s2(E.e1, p2((xx + yy) + xy, (xx + yy) - xy));
+    E.e2 = s2(E.e2, p2((xx + zz) + xz, (xx + zz) - xz));
+    E.e3 = s2(E.e3, p2((yy + zz) + yz, (yy + zz) - yz));
+    E.f1 = s2(E.f1, p2(xx, yy));
+    E.f5 -= zz;
+  }
+  const float r3 = 3.0f * c.r, r9 = 9.0f * c.r;   // 2 * 4.5 r
+  const AdjPairs cv = along(c.vx, c.vy, c.vz);
+  const float2 cE1 = m2(cv.e1, E.e1), cE2 = m2(cv.e2, E.e2), cE3 = m2(cv.e3, E.e3),
+               cF1 = m2(cv.f1, E.f1);
+  const float cF5 = cv.f5 * E.f5;
+  // sums over the edges and the faces of E, c G and c^2 E
+  const float2 eE = a2(a2(E.e1, E.e2), E.e3);
+  const float2 eG = fm2(cv.e3, G.e3, fm2(cv.e2, G.e2, m2(cv.e1, G.e1)));
+  const float2 eC = fm2(cv.e3, cE3, fm2(cv.e2, cE2, m2(cv.e1, cE1)));
+  const float2 fG = m2(cv.f1, G.f1), fC = m2(cv.f1, cF1);
+  const float Ab = W0 * e0 + WE * (eE.x + eE.y) + WF * ((E.f1.x + E.f1.y) + E.f5);
+  const float r3b = WE * (eG.x + eG.y) + WF * ((fG.x + fG.y) + cv.f5 * G.f5);
+  const float r45b = WE * (eC.x + eC.y) + WF * ((fC.x + fC.y) + cv.f5 * cF5);
+  // adjoint of c_a . u per pair: w (3 r G + 9 r c E)
+  const float2 wr3e = p2(WE * r3), wr9e = p2(WE * r9), wr3f = p2(WF * r3), wr9f = p2(WF * r9);
+  const AdjPairs cb{fm2(wr3e, G.e1, m2(wr9e, cE1)), fm2(wr3e, G.e2, m2(wr9e, cE2)),
+                    fm2(wr3e, G.e3, m2(wr9e, cE3)), fm2(wr3f, G.f1, m2(wr9f, cF1)),
+                    fmaf(WF * r3, G.f5, WF * r9 * cF5)};
+  float vxb, vyb, vzb;
+  moment(cb, vxb, vyb, vzb);
+  const float usqb = -(1.5f * c.r * Ab);
+  vxb = fmaf(2.0f * c.vx, usqb, vxb);
+  vyb = fmaf(2.0f * c.vy, usqb, vyb);
+  vzb = fmaf(2.0f * c.vz, usqb, vzb);
+  invb += vxb * c.jx + vyb * c.jy + vzb * c.jz;
+  const float rb = 3.0f * r3b + 4.5f * r45b - 1.5f * c.usq * Ab - c.inv * c.inv * invb;
+  const float drb = Ab + rb;
+  const AdjPairs cj = along(vxb * c.inv, vyb * c.inv, vzb * c.inv);
+  out(0, (ab[0] - e0) + drb);
+  const float2 mh = p2(-0.5f), drb2 = p2(drb);
+  auto pair2 = [&](int q, float2 x, float2 y, float2 e, float2 g, float2 j) {
+    const float2 h = fm2(mh, e, drb2), k = fm2(mh, g, j);
+    const float2 va = a2(x, a2(h, k)), vb = a2(y, s2(h, k));
+    out(q, va.x); out(q + 1, vb.x); out(q + 2, va.y); out(q + 3, vb.y);
+  };
+  pair2(7, ga.e1, gb.e1, E.e1, G.e1, cj.e1);
+  pair2(11, ga.e2, gb.e2, E.e2, G.e2, cj.e2);
+  pair2(15, ga.e3, gb.e3, E.e3, G.e3, cj.e3);
+  pair2(1, ga.f1, gb.f1, E.f1, G.f1, cj.f1);
+  const float h5 = fmaf(-0.5f, E.f5, drb), k5 = fmaf(-0.5f, G.f5, cj.f5);
+  out(5, ga.f5 + (h5 + k5));
+  out(6, gb.f5 + (h5 - k5));
+}
+
 // One adjoint step, one thread per cell. A computed cell recomputes its
 // forward collision from the stored state, gathers the adjoints of the 19
 // populations it stored (the consumers of its links in the next step), runs
@@ -500,11 +610,15 @@ __device__ __forceinline__ T adj_shell(const StepArgs<S>& a, const T* Tn, int q,
 // NB: offsets in bytes (every buffer spans < 2^31 bytes) instead of 64-bit
 // element indices.
 // Resident blocks per SM the register budget is set for, the fastest measured
-// on B200: float32 adjoints of a half-storage state 5 (96 registers; 4
-// measured 7% slower), of a float32 state 4 (128 registers, no spills; 3%
-// faster than 5); float64 adjoints 3 (168 registers).
+// on B200 (backward sweep, recomputation included, microseconds a step by number
+// of blocks): float32 adjoints of a half-storage state (384x160x160) 4: 626, 5: 589,
+// 6: 566; of a float32 state (128x64x64) 4: 37.6, 5: 36.1, 6: 39.4; one pair of
+// directions per instruction, 5 and 4 blocks: 652 and 41.6. Gathering after the
+// forward collision instead of with the pulls spills (702 and 40.8). Float64
+// adjoints 3 (168 registers). Bound by memory latency: 190 bytes per cell of a half
+// state at 0.8 of the measured copy rate.
 template <class S, class T>
-constexpr int adj_min_blocks() { return sizeof(T) == 8 ? 3 : (sizeof(S) == 4 ? 4 : 5); }
+constexpr int adj_min_blocks() { return sizeof(T) == 8 ? 3 : (sizeof(S) == 4 ? 5 : 6); }
 
 template <class S, class T, bool NB>
 __global__ void __launch_bounds__(STEP_BX, adj_min_blocks<S, T>()) k_adjoint(const __grid_constant__ StepArgs<S> a,
@@ -608,54 +722,107 @@ __global__ void __launch_bounds__(STEP_BX, adj_min_blocks<S, T>()) k_adjoint(con
     for (int q = 0; q < Q; q++)
       if ((sm >> q) & 1u) c.f[q] = f_own(opp(q));
   }
-  cell_fw<T>(a, c);
   const T wJ = (T)j.wJ;
-  // partial bounce-back: g = (1-s) gc + s f_opp, force s sum_q c_q (gc_q - f_opp(q))
-  T st = (T)0;
-  if (a.sfrac && x >= a.sb[0] && x < a.sb[3] && y >= a.sb[1] && y < a.sb[4] && z >= a.sb[2] &&
-      z < a.sb[5]) {
-    st = (T)sfrac_at(a, x, y, z);
-    // dJ/ds = sum_q g_q (f_opp(q) - gc_q) + wJ sum_q c_q (gc_q - f_opp(q))
-    T g1 = (T)0, g2 = (T)0;
+  const bool box = a.sfrac && x >= a.sb[0] && x < a.sb[3] && y >= a.sb[1] && y < a.sb[4] &&
+                   z >= a.sb[2] && z < a.sb[5];
+  double* const ds = j.ds + ((x - a.sb[0]) + (long long)(a.sb[3] - a.sb[0]) *
+                                                 ((y - a.sb[1]) + (long long)(a.sb[4] - a.sb[1]) *
+                                                                      (z - a.sb[2])));
+  if constexpr (std::is_same<T, float>::value) {
+    AdjCell k;
+    adj_forward(a, c.f, k);
+    // what the blend, the force and the body links add to the pulled values'
+    // adjoints goes through this thread's column of shared memory (its free-slip
+    // terms have been taken), so that the common path carries nothing for it
+    const bool extra = box || om;
+    if (extra) {
+      T st = (T)0;
+      if (box) {
+        st = (T)sfrac_at(a, x, y, z);
+        // dJ/ds = sum_q g_q (f_opp(q) - gc_q) + wJ sum_q c_q (gc_q - f_opp(q))
+        T g1 = g[0] * (k.om * k.n0), g2 = (T)0;
+        const AdjPairs cv = along(k.vx, k.vy, k.vz);
+        auto link = [&](int q, T sp, T sm, T c_) {
+          // f_a - f_b of the pair, from sm: the pulled values are not kept
+          const T d = 2.0f * fmaf((float)wq(q) * 3.0f * k.r, c_, sm);
+          const T da = k.om * sp + k.omm * sm - d, db = k.om * sp - k.omm * sm + d;
+          const T cc = (T)(j.comp == 0 ? ex(q) : (j.comp == 1 ? ey(q) : ez(q)));
+          g1 += g[q] * da + g[q + 1] * db;
+          g2 -= cc * (da - db);
+        };
+        link(1, k.sp.f1.x, k.sm.f1.x, cv.f1.x); link(3, k.sp.f1.y, k.sm.f1.y, cv.f1.y);
+        link(5, k.sp.f5, k.sm.f5, cv.f5);
+        link(7, k.sp.e1.x, k.sm.e1.x, cv.e1.x); link(9, k.sp.e1.y, k.sm.e1.y, cv.e1.y);
+        link(11, k.sp.e2.x, k.sm.e2.x, cv.e2.x); link(13, k.sp.e2.y, k.sm.e2.y, cv.e2.y);
+        link(15, k.sp.e3.x, k.sm.e3.x, cv.e3.x); link(17, k.sp.e3.y, k.sm.e3.y, cv.e3.y);
+        *ds += (double)(g1 + wJ * g2);
+      }
+      const T ws = wJ * st, s1 = (T)1 - st;
+      auto cell = [&](int q, T ga, T go) {   // g_q and g_opp(q)
+        const T cc = (T)(j.comp == 0 ? ex(q) : (j.comp == 1 ? ey(q) : ez(q)));
+        T e = st * go + ws * cc;
+        if ((om >> q) & 1u) e -= (T)2 * wJ * cc;   // momentum exchange of a body link
+        mir[q][threadIdx.x] = e;
+        return st != (T)0 ? s1 * ga + ws * cc : ga;
+      };
+      g[0] = cell(0, g[0], g[0]);
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const T cc = (T)(j.comp == 0 ? ex(q) : (j.comp == 1 ? ey(q) : ez(q)));
-      const T d = c.f[opp(q)] - c.gc[q];
-      g1 += g[q] * d;
-      g2 -= cc * d;
+      for (int q = 1; q < Q; q += 2) {
+        const T ga = g[q], gb = g[q + 1];
+        g[q] = cell(q, ga, gb);
+        g[q + 1] = cell(q + 1, gb, ga);
+      }
     }
-    j.ds[(x - a.sb[0]) + (long long)(a.sb[3] - a.sb[0]) *
-                             ((y - a.sb[1]) + (long long)(a.sb[4] - a.sb[1]) * (z - a.sb[2]))] +=
-        (double)(g1 + wJ * g2);
-  }
-  // adjoints of the collided values (ab) and, through the blend and the
-  // force, of the pulled ones (fb); s = 0 leaves ab = g, fb = 0
-  T ab[Q], fb[Q];
-  if (st != (T)0) {
-    const T ws = wJ * st, s1 = (T)1 - st;
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const T cc = (T)(j.comp == 0 ? ex(q) : (j.comp == 1 ? ey(q) : ez(q)));
-      ab[q] = s1 * g[q] + ws * cc;
-      fb[q] = st * g[opp(q)] + ws * cc;
-    }
+    adj_backward(a, k, g, [&](int q, T v) {
+      if (extra) v += mir[q][threadIdx.x];
+      trow(Tci, q) = v;
+    });
   } else {
+    cell_fw<T>(a, c);
+    // partial bounce-back: g = (1-s) gc + s f_opp, force s sum_q c_q (gc_q - f_opp(q))
+    T st = (T)0;
+    if (box) {
+      st = (T)sfrac_at(a, x, y, z);
+      // dJ/ds = sum_q g_q (f_opp(q) - gc_q) + wJ sum_q c_q (gc_q - f_opp(q))
+      T g1 = (T)0, g2 = (T)0;
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      ab[q] = g[q];
-      fb[q] = (T)0;
+      for (int q = 0; q < Q; q++) {
+        const T cc = (T)(j.comp == 0 ? ex(q) : (j.comp == 1 ? ey(q) : ez(q)));
+        const T d = c.f[opp(q)] - c.gc[q];
+        g1 += g[q] * d;
+        g2 -= cc * d;
+      }
+      *ds += (double)(g1 + wJ * g2);
     }
-  }
-  if (om) {
+    // adjoints of the collided values (ab) and, through the blend and the
+    // force, of the pulled ones (fb); s = 0 leaves ab = g, fb = 0
+    T ab[Q], fb[Q];
+    if (st != (T)0) {
+      const T ws = wJ * st, s1 = (T)1 - st;
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const T cc = (T)(j.comp == 0 ? ex(q) : (j.comp == 1 ? ey(q) : ez(q)));
-      if ((om >> q) & 1u) fb[q] -= (T)2 * wJ * cc;   // momentum exchange of a body link
+      for (int q = 0; q < Q; q++) {
+        const T cc = (T)(j.comp == 0 ? ex(q) : (j.comp == 1 ? ey(q) : ez(q)));
+        ab[q] = s1 * g[q] + ws * cc;
+        fb[q] = st * g[opp(q)] + ws * cc;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        ab[q] = g[q];
+        fb[q] = (T)0;
+      }
     }
-  }
-  cell_vjp<T>(a, c, ab, fb);
+    if (om) {
 #pragma unroll
-  for (int q = 0; q < Q; q++) trow(Tci, q) = fb[q];
+      for (int q = 0; q < Q; q++) {
+        const T cc = (T)(j.comp == 0 ? ex(q) : (j.comp == 1 ? ey(q) : ez(q)));
+        if ((om >> q) & 1u) fb[q] -= (T)2 * wJ * cc;   // momentum exchange of a body link
+      }
+    }
+    cell_vjp<T>(a, c, ab, fb);
+#pragma unroll
+    for (int q = 0; q < Q; q++) trow(Tci, q) = fb[q];
+  }
 }
 
 // Launch one adjoint step (both kernels' offset forms are instantiated by the
