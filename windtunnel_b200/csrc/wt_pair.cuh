@@ -443,7 +443,7 @@ template <class S, bool SR, int MODE, bool BLEND>
 __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
                                                    typename PairIO<S>::W (&w)[Q],
                                                    long long i0, const PairCells& cells,
-                                                   f2 sf, f2 (&F)[3]) {
+                                                   bool special_warp, f2 sf, f2 (&F)[3]) {
   using IO = PairIO<S>;
   using W = typename IO::W;
   using R = typename IO::R;
@@ -685,6 +685,9 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
   uint32_t h = 0, h1 = 0;
   if constexpr (SR) h = mix(i0);
   if constexpr (SR && REF) h1 = mix(i0 + 1);
+  // pass 2, written twice: `special` warps hold a solid cell, whose pair stores
+  // the other cell alone; in the others a store is one permute and one store
+  auto outputs = [&](auto special) {
   auto store = [&](int q, W v) {
     // the inlet's low cell takes the equilibrium, the outlet's high cell
     // takes cell nx-2's value
@@ -693,7 +696,7 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
       if (!keep0) gh(q, 0) = IO::lane(v, 0);
       if (!keep1) gh(q, 1) = IO::lane(v, 1);
       if (cells.dup && !keep1) gh(q, 2) = IO::lane(v, 1);
-    } else if (!keep_any) {
+    } else if (!decltype(special)::value || !keep_any) {
       gw(q) = v;
     } else {
       // a solid cell of the pair keeps its stale population
@@ -777,6 +780,11 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     WT_PAIR_OUT(17, psub(vy, vz), k45e, kae, k3e)
 #undef WT_PAIR_OUT
   }
+  };
+  // float32 storage is bound by memory and runs 0.4% slower with two copies
+  constexpr bool TWICE = sizeof(R) == 2 || BLEND || MOV || (MODE & PAIR_PBB) != 0;
+  if (!TWICE || special_warp) outputs(std::true_type{});
+  else outputs(std::false_type{});
   if (outlet && solid0) {
     // copy of a solid cell nx-2, whose g this step does not write
     R v[Q];
@@ -877,6 +885,7 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
     pair_force_partial(Fx * inv_sc, Fy * inv_sc, Fz * inv_sc,
                        (active && (c.near0 || c.near1)) || in_box, a, seg);
   }
+  const bool special = __any_sync(0xffffffffu, c.solid0 || c.solid1);
   f2 sf = pk(0.0f), F[3] = {pk(0.0f), pk(0.0f), pk(0.0f)};
   const bool blend = PBB && __any_sync(0xffffffffu, in_box);
   if (PBB && blend && in_box) {
@@ -884,9 +893,9 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
     if (c.fluid1) sf.y = (float)sfrac_at(a, x0 + 1, y, z);
   }
   if (blend) {
-    if (active) pair_collide_store<S, SR, MODE, PBB>(a, w, i0, c, sf, F);
+    if (active) pair_collide_store<S, SR, MODE, PBB>(a, w, i0, c, special, sf, F);
   } else {
-    if (active) pair_collide_store<S, SR, MODE, false>(a, w, i0, c, sf, F);
+    if (active) pair_collide_store<S, SR, MODE, false>(a, w, i0, c, special, sf, F);
   }
   if (PBB && blend) {
     // the blend's force joins the partial that this half-warp's first lane stored
