@@ -159,6 +159,9 @@ struct StepArgs {
   const double* sfrac; // partial bounce-back: solid fraction on the box sb (x fastest), or null
   int sb[6];           // its half-open box x0, y0, z0, x1, y1, z1
   long long pf;        // L2 prefetch distance in cells (0: none), see prefetch_ahead
+  // pair kernel: F + src[q] and G + dst[q], set by its launcher
+  const char* fq[Q];
+  char* gq[Q];
 };
 
 // Ask L2 for the populations that the warp pf cells further on in launch

@@ -89,7 +89,12 @@ cudaError_t each_pair_kernel(F f) {
 template <class S>
 void launch_pair(const StepArgs<S>& a, cudaStream_t s) {
   const int mode = pair_mode(a);
-  launch_pdl(pair_kernel<S>(a.f16_sr != 0, mode), pair_grid(a, mode), dim3(PAIR_BX), s, a);
+  StepArgs<S> b = a;
+  for (int q = 0; q < Q; q++) {
+    b.fq[q] = reinterpret_cast<const char*>(a.F + a.src[q]);
+    b.gq[q] = reinterpret_cast<char*>(a.G + a.dst[q]);
+  }
+  launch_pdl(pair_kernel<S>(a.f16_sr != 0, mode), pair_grid(a, mode), dim3(PAIR_BX), s, b);
 }
 
 void launch_pair_f16(const StepArgs<__half>& a, dim3, bool, cudaStream_t s) { launch_pair(a, s); }

@@ -88,6 +88,13 @@ constexpr int pair_arith(int mode) {
                          : (mode & PAIR_MOV ? ARITH_DIRECT : (mode & PAIR_ODD ? ARITH_LEAN : ARITH_OWN));
 }
 
+// Addresses: a uniform pointer per direction plus one 32-bit offset per thread
+// (half storage, whose plain step is bound by issue and latency: 512x192x192 282 ->
+// 275 us a step on B200), else one pointer per thread plus a uniform offset
+// (float32: the same within 0.5%, moving walls 1% slower the other way).
+template <class S>
+constexpr bool pair_uniform(int mode) { return sizeof(S) == 2 && !(mode & PAIR_PBB); }
+
 template <class S>
 constexpr int pair_min_blocks(int mode) {
   if (mode & PAIR_PBB) return 4;
@@ -449,13 +456,17 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
   using R = typename IO::R;
   constexpr float SC = IO::SC;
   constexpr bool ODD = (MODE & PAIR_ODD) != 0, MOV = (MODE & PAIR_MOV) != 0;
+  constexpr bool FQ = pair_uniform<S>(MODE);
   const bool inlet = cells.inlet, outlet = cells.outlet, solid0 = cells.solid0,
              solid1 = cells.solid1, fluid0 = cells.fluid0, fluid1 = cells.fluid1;
   char* Gb = reinterpret_cast<char*>(a.G + i0);
-  auto gw = [&](int q) -> W& { return *reinterpret_cast<W*>(Gb + a.dstb[q]); };
-  auto gh = [&](int q, int L) -> R& {
-    return *reinterpret_cast<R*>(Gb + a.dstb[q] + sizeof(R) * L);
+  const uint32_t at = (uint32_t)((unsigned long long)i0 * sizeof(S));
+  auto gp = [&](int q) -> char* {
+    if constexpr (FQ) return a.gq[q] + at;
+    else return Gb + a.dstb[q];
   };
+  auto gw = [&](int q) -> W& { return *reinterpret_cast<W*>(gp(q)); };
+  auto gh = [&](int q, int L) -> R& { return *reinterpret_cast<R*>(gp(q) + sizeof(R) * L); };
   // ---- pass 1: moments --------------------------------------------------
   constexpr int AR = pair_arith(MODE);
   constexpr bool REF = AR != ARITH_OWN;
@@ -687,6 +698,8 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
   if constexpr (SR && REF) h1 = mix(i0 + 1);
   // pass 2, written twice: `special` warps hold a solid cell, whose pair stores
   // the other cell alone; in the others a store is one permute and one store
+  // float32 storage is bound by memory and runs 0.4% slower with two copies
+  constexpr bool TWICE = sizeof(R) == 2 || BLEND || MOV || (MODE & PAIR_PBB) != 0;
   auto outputs = [&](auto special) {
   auto store = [&](int q, W v) {
     // the inlet's low cell takes the equilibrium, the outlet's high cell
@@ -781,8 +794,6 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
 #undef WT_PAIR_OUT
   }
   };
-  // float32 storage is bound by memory and runs 0.4% slower with two copies
-  constexpr bool TWICE = sizeof(R) == 2 || BLEND || MOV || (MODE & PAIR_PBB) != 0;
   if (!TWICE || special_warp) outputs(std::true_type{});
   else outputs(std::false_type{});
   if (outlet && solid0) {
@@ -840,11 +851,13 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
   // L2 prefetch of the populations the warp a fixed distance ahead will
   // pull (StepArgs pf; set for half storage on lattices within twice the L2)
   prefetch_ahead(a, i0 - 2 * (long long)(threadIdx.x & 31));
+  constexpr bool FQ = pair_uniform<S>(MODE);
+  const uint32_t at = (uint32_t)((unsigned long long)i0 * sizeof(S));
   const char* Fb = reinterpret_cast<const char*>(a.F + i0);
   typename IO::Raw raw[Q];
   if (active) {
     // byte address of the source of cell x0
-#define WT_PAIR_PULL(q) raw[q] = IO::template load<ex(q), ODD>(Fb + a.srcb[q]);
+#define WT_PAIR_PULL(q) raw[q] = IO::template load<ex(q), ODD>(FQ ? a.fq[q] + at : Fb + a.srcb[q]);
 #define WT_PAIR_SHELL(q)                 \
   raw[q] = IO::template load<ex(q), ODD>( \
       reinterpret_cast<const char*>(a.F + (i0 + shell_src<q>(a, row))));
