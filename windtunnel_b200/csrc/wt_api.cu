@@ -195,7 +195,7 @@ wt::StepArgs<S> make_args(wt_lattice* h) {
   }
   a.sfrac = h->sfrac;
   for (int k = 0; k < 6; k++) a.sb[k] = h->sbox[k];
-  a.pf = h->pf;   // read by the lean kernel only
+  a.pf = h->pf;
   return a;
 }
 
@@ -241,8 +241,8 @@ bool pair_auto(const wt_lattice* h);
 
 // The kernel WT_KERNEL_AUTO runs, the fastest measured on B200 for the form
 // (256x128x128 channel, 1000-step calls): the pair kernel where it can run
-// (float32 storage 40.3k MLUPS against 37.9k for the lean kernel; half
-// storage 55.2k against 44.4k; odd nx and moving walls: PAIR_ODD, PAIR_MOV),
+// (float32 storage 43.0k MLUPS against 37.9k for the lean kernel; half
+// storage 66k against 44.4k; odd nx and moving walls: PAIR_ODD, PAIR_MOV),
 // the lean kernel for half storage with an odd nx, the direct kernel otherwise
 // (exact collision, float64, half storage with moving walls, buffers of 2^31
 // bytes or more).
@@ -253,9 +253,7 @@ Path auto_path(const wt_lattice* h) {
 }
 
 // True when the lean-addressing kernel can run.
-// Moving walls are excluded: their correction reads the previous step's
-// density, which the thread of cell nx-2 rewrites while the outlet thread
-// recomputes that cell.
+// Moving walls are excluded: it has no wall-speed correction.
 bool lean_ok(const wt_lattice* h) {
   const bool exact = h->p.math == WT_MATH_EXACT || h->storage == WT_STORE_F64;
   return !exact && !h->p.moving_walls && 19 * h->n * (long long)h->elem < (1LL << 31);

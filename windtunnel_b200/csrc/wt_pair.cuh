@@ -53,8 +53,9 @@ namespace wt {
 // spills, 24 warps; 64-thread blocks 1.5% slower). The variants' figures,
 // microseconds a step by number of blocks: odd nx (193x85x91) 4: 41.3, 5: 41.9, 6:
 // 54; moving walls (160x80x80 over a road) 4: 32.1, 5: 29.3, 6: 32.0; partial
-// bounce-back float32 (128x64x64, a 32^3 box) 3: 15.3, 4: 13.3, 5: 14.5, half storage
-// (384x160x160, a 64^3 box) 4: 239, 5: 244, 6: 266.
+// bounce-back float32 (128x64x64, a 32^3 box) 3: 15.3, 4: 13.3, 5: 14.5 (now 12.7 at
+// 4), half storage (384x160x160, a 64^3 box) 4: 218, 5: 234, 6: 240; half storage
+// (256x128x128, stochastic rounding) 6: 65.2, 7: 63.3, 8: 67.7.
 constexpr int PAIR_BX = 128;
 
 // Variants of the pair kernel. ODD: an odd nx (float32 storage only): pairs
@@ -68,8 +69,8 @@ constexpr int PAIR_BX = 128;
 // partial bounce-back field (wt_pbb.cuh): the blend of a box cell's outputs with
 // its reversed inputs, and its force.
 // Measured on B200, microseconds a step, one-cell kernel / pair kernel: 193x85x91
-// float32 46.3 / 41.3 (ODD against lean); 160x80x80 float32 over a rolling road
-// 40.3 / 29.3 (MOV against direct); PBB float32 18.5 / 13.3, half storage 289 / 239. Pairs
+// float32 46.3 / 41.5 (ODD against lean); 160x80x80 float32 over a rolling road
+// 40.3 / 28.8 (MOV against direct); PBB float32 18.5 / 12.7, half storage 289 / 218. Pairs
 // across row ends against one row per block: 64x32x32 float32 8.2 / 6.7 us (three of
 // a block's four warps had nothing to do); on 256x128x128 and 512x192x192 one row
 // per block is 1-2% faster for half storage.
@@ -156,17 +157,15 @@ struct PairIO<__half> {
   // (x0+1, x0+2) the word at p-2 and the half at p+2. Loading and joining are
   // apart so that a branch around the loads does not wait for them.
   struct Raw { uint32_t w, h; };
-  template <int dx, bool ODD>
+  template <int dx, bool>
   __device__ __forceinline__ static Raw load(const char* p) {
-    if constexpr (ODD) return Raw{ld16(p), ld16(p + 2)};
-    else if constexpr (dx == 0) return Raw{ld32(p), 0u};
+    if constexpr (dx == 0) return Raw{ld32(p), 0u};
     else if constexpr (dx == 1) return Raw{ld32(p + 2), ld16(p)};
     else return Raw{ld32(p - 2), ld16(p + 2)};
   }
-  template <int dx, bool ODD>
+  template <int dx>
   __device__ __forceinline__ static W join(const Raw& r) {
-    if constexpr (ODD) return prmt(r.w, r.h, 0x5410u);
-    else if constexpr (dx == 0) return r.w;
+    if constexpr (dx == 0) return r.w;
     else if constexpr (dx == 1) return prmt(r.h, r.w, 0x5410u);
     else return prmt(r.w, r.h, 0x5432u);
   }
@@ -174,9 +173,6 @@ struct PairIO<__half> {
   __device__ __forceinline__ static f2 to_f2(W w) { return h2f(w); }
   __device__ __forceinline__ static W pack(f2 g) { return f2h(g); }
   __device__ __forceinline__ static W pack_sr(f2 g, uint32_t r) { return f2h_sr(g, r); }
-  // words of the high / low halves of two words
-  __device__ __forceinline__ static W highs(W x, W y) { return prmt(x, y, 0x7632u); }
-  __device__ __forceinline__ static W lows(W x, W y) { return prmt(x, y, 0x5410u); }
   __device__ __forceinline__ static W eq(const StepArgs<__half>& a, int q) { return a.eq2[q]; }
   __device__ __forceinline__ static W fix(W v, W e, bool inlet, bool outlet) {
     return prmt(v, e, inlet ? 0x3254u : (outlet ? 0x1010u : 0x3210u));
@@ -203,14 +199,11 @@ struct PairIO<float> {
     if constexpr (dx == 0 && !ODD) return *reinterpret_cast<const float2*>(p);
     else return make_float2(*reinterpret_cast<const float*>(p), *reinterpret_cast<const float*>(p + 4));
   }
-  template <int dx, bool ODD>
+  template <int dx>
   __device__ __forceinline__ static W join(const Raw& r) { return r; }
   __device__ __forceinline__ static void opaque(W& w) { asm volatile("" : "+f"(w.x), "+f"(w.y)); }
   __device__ __forceinline__ static f2 to_f2(W w) { return w; }
   __device__ __forceinline__ static W pack(f2 g) { return g; }
-  __device__ __forceinline__ static W pack_sr(f2 g, uint32_t) { return g; }
-  __device__ __forceinline__ static W highs(W x, W y) { return make_float2(x.y, y.y); }
-  __device__ __forceinline__ static W lows(W x, W y) { return make_float2(x.x, y.x); }
   __device__ __forceinline__ static W eq(const StepArgs<float>& a, int q) {
     return make_float2(a.eq[q], a.eq[q]);
   }
@@ -682,23 +675,17 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
   const bool keep0 = solid0 && !inlet, keep1 = solid1 || (outlet && solid0);
   const bool keep_any = keep0 || keep1;
   // stochastic rounding: a hash of (pair, step), then per output word its
-  // product with a distinct odd constant (one multiply per word); REF: the
-  // one-cell kernels' chain of each of the two cells, 32 bits per opposite pair
-  auto mix = [&](long long i) {
-    uint32_t v = ((uint32_t)i ^ (uint32_t)(i >> 32)) * 0x9E3779B1u ^ a.sr_seed;
-    v ^= v >> 16; v *= 0x85EBCA6Bu; v ^= v >> 13; v *= 0xC2B2AE35u; v ^= v >> 16;
-    return v;
-  };
-  auto next = [](uint32_t v) {
-    v ^= v << 13; v ^= v >> 17; v ^= v << 5;
-    return v;
-  };
-  uint32_t h = 0, h1 = 0;
-  if constexpr (SR) h = mix(i0);
-  if constexpr (SR && REF) h1 = mix(i0 + 1);
-  // pass 2, written twice: `special` warps hold a solid cell, whose pair stores
+  // product with a distinct odd constant (one multiply per word)
+  static_assert(!(SR && REF), "stochastic rounding: the plain variants only");
+  uint32_t h = 0;
+  if constexpr (SR) {
+    h = ((uint32_t)i0 ^ (uint32_t)(i0 >> 32)) * 0x9E3779B1u ^ a.sr_seed;
+    h ^= h >> 16; h *= 0x85EBCA6Bu; h ^= h >> 13; h *= 0xC2B2AE35u; h ^= h >> 16;
+  }
+  // Pass 2, written twice: `special` warps hold a solid cell, whose pair stores
   // the other cell alone; in the others a store is one permute and one store
-  // float32 storage is bound by memory and runs 0.4% slower with two copies
+  // (half storage 512x192x192 303 -> 282 us a step on B200; plain float32 storage
+  // is bound by memory and 0.4% slower with two copies).
   constexpr bool TWICE = sizeof(R) == 2 || BLEND || MOV || (MODE & PAIR_PBB) != 0;
   auto outputs = [&](auto special) {
   auto store = [&](int q, W v) {
@@ -721,18 +708,6 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     if constexpr (SR) store(q, IO::pack_sr(g, h * (0x9E3779B1u * (2u * (uint32_t)q + 1u))));
     else store(q, IO::pack(g));
   };
-  auto put2 = [&](int q, f2 ga, f2 gb) {   // the pair (q, q+1)
-    if constexpr (SR && REF) {
-      h = next(h);
-      h1 = next(h1);
-      const W x = IO::pack_sr(make_float2(gb.x, ga.x), h), y = IO::pack_sr(make_float2(gb.y, ga.y), h1);
-      store(q, IO::highs(x, y));
-      store(q + 1, IO::lows(x, y));
-    } else {
-      put(q, ga);
-      put(q + 1, gb);
-    }
-  };
   // ---- pass 2: outputs ----------------------------------------------------
   const f2 s1 = psub(pk(1.0f), sf);   // BLEND only
   if constexpr (REF) {
@@ -754,7 +729,8 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
         ga = pfma(sf, fb, pmul(s1, ga));
         gb = pfma(sf, fa, pmul(s1, gb));
       }
-      put2(q, ga, gb);
+      put(q, ga);
+      put(q + 1, gb);
     };
     out(1, vx); out(3, vy); out(5, vz);
     out(7, padd(vx, vy)); out(9, psub(vx, vy)); out(11, padd(vx, vz));
@@ -762,13 +738,7 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     const f2 f0 = IO::to_f2(w[0]);
     f2 g0 = pfma(nom, pfma(pk(-W0), A, f0), f0);
     if constexpr (BLEND) g0 = pfma(sf, f0, pmul(s1, g0));
-    if constexpr (SR) {
-      h = next(h);
-      h1 = next(h1);
-      store(0, IO::lows(IO::pack_sr(make_float2(g0.x, 0.0f), h), IO::pack_sr(make_float2(g0.y, 0.0f), h1)));
-    } else {
-      store(0, IO::pack(g0));
-    }
+    put(0, g0);
   } else {
     const f2 f0 = IO::to_f2(w[0]);
     put(0, pfma(pfma(pk(-1.0f), om, pk(1.0f)), f0, pmul(pk((float)(1.0 / 3)), omA)));
@@ -780,7 +750,8 @@ __device__ __forceinline__ void pair_collide_store(const StepArgs<S>& a,
     const f2 X = pfma(pmul(c, c), K45, KA);                         \
     const f2 Y = pmul(K3, c);                                       \
     const f2 P = pfma(al, s, X), M = pfma(be, d, Y);                \
-    put2(qa, padd(P, M), psub(P, M));                               \
+    put(qa, padd(P, M));                                            \
+    put(qa + 1, psub(P, M));                                        \
   }
     WT_PAIR_OUT(1, vx, k45f, kaf, k3f)
     WT_PAIR_OUT(3, vy, k45f, kaf, k3f)
@@ -876,7 +847,7 @@ __global__ void __launch_bounds__(PAIR_BX, pair_min_blocks<S>(MODE))
     else fl = ld16(reinterpret_cast<const char*>(a.flags + i0));
   }
   W w[Q];
-#define WT_PAIR_JOIN(q) w[q] = IO::template join<ex(q), ODD>(raw[q]);
+#define WT_PAIR_JOIN(q) w[q] = IO::template join<ex(q)>(raw[q]);
   WT_EACH_Q(WT_PAIR_JOIN)
 #undef WT_PAIR_JOIN
   const PairCells c = pair_cells<MODE>(fl, x0, a.nx);

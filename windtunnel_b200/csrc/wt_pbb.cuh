@@ -612,8 +612,9 @@ __device__ __forceinline__ void adj_backward(const StepArgs<S>& a, const AdjCell
 // Resident blocks per SM the register budget is set for, the fastest measured
 // on B200 (backward sweep, recomputation included, microseconds a step by number
 // of blocks): float32 adjoints of a half-storage state (384x160x160) 4: 626, 5: 589,
-// 6: 566; of a float32 state (128x64x64) 4: 37.6, 5: 36.1, 6: 39.4; one pair of
-// directions per instruction, 5 and 4 blocks: 652 and 41.6. Gathering after the
+// 6: 566 (551 with the recomputation's present step); of a float32 state (128x64x64)
+// 4: 37.6, 5: 36.1, 6: 39.4; one pair of directions per instruction, 5 and 4 blocks: 652
+// and 41.6. Gathering after the
 // forward collision instead of with the pulls spills (702 and 40.8). Float64
 // adjoints 3 (168 registers). Bound by memory latency: 190 bytes per cell of a half
 // state at 0.8 of the measured copy rate.
